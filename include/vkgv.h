@@ -416,6 +416,10 @@ enum {
 };
 /* Captures the selected passes over these views into one CUDA graph (a
  * training step: zero, forward, backward), launched with vkgv_graph_launch.
+ * A step of both FORWARD and BACKWARD is recorded as one pass that
+ * recomputes the visibility and writes images and gradients, with the results
+ * of the two in order (two passes where an image overlaps a buffer that the
+ * backward pass reads).
  * Pointers, sizes, scale and view count are baked in; parameter, camera and
  * target contents may change between launches. */
 int vkgv_diff_graph_capture(vkgv_ctx* ctx, const vkgv_diff_scene* scene, const vkgv_diff_view* views,

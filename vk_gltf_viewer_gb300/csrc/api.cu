@@ -996,6 +996,53 @@ int diff_prepare(vkgv_ctx* ctx, const vkgv_diff_scene* ds, const vkgv_diff_view*
     return VKGV_OK;
 }
 
+// Whether the backward pass of a captured step may write the forward images
+// as it shades: nothing that it reads (or the step writes elsewhere) may lie
+// in an image, since in the two-pass order every image is complete before
+// the backward pass reads anything (an image handed in as its own dL/drgb,
+// for instance).  Images may overlap each other: both orders race alike.
+bool one_pass_step(const vkgv_diff_scene& S, const vkgv_diff_view* views, uint32_t n, uint64_t loss, uint64_t gpos,
+                   uint64_t gcol, uint64_t gtex) {
+    struct Span {
+        uint64_t lo, hi;
+        bool image;
+    };
+    std::vector<Span> spans;
+    spans.reserve(5 * (size_t)n + 16);
+    auto add = [&](uint64_t at, uint64_t bytes, bool image) {
+        if (at && bytes) spans.push_back(Span{at, at + bytes, image});
+    };
+    for (uint32_t i = 0; i < n; ++i) {
+        const vkgv_diff_view& v = views[i];
+        const uint64_t px = (uint64_t)v.width * v.height;
+        add(v.rgb, 12 * px, true);
+        add(v.target, 12 * px, false);
+        add(v.grad_rgb, 12 * px, false);
+        add(v.depth_id, 8 * px, false);
+        add(v.camera_buffer, sizeof(vkgv_camera), false);
+    }
+    const uint64_t V = S.vertex_count, T = (uint64_t)S.tex_width * S.tex_height;
+    add(S.positions, 12 * V, false);
+    add(S.colors, 12 * V, false);
+    add(S.uvs, 8 * V, false);
+    add(S.texture, 12 * T, false);
+    add(S.meshlet_buffer, sizeof(vkgv_meshlet) * (uint64_t)S.meshlet_count, false);
+    add(S.vertex_index_buffer, 4, false);     // lengths unknown: their first bytes
+    add(S.primitive_index_buffer, 1, false);
+    add(loss, 4, false);
+    add(gpos, 12 * V, false);
+    add(gcol, 12 * V, false);
+    add(gtex, 12 * T, false);
+    std::sort(spans.begin(), spans.end(), [](const Span& a, const Span& b) { return a.lo < b.lo; });
+    uint64_t image_end = 0, other_end = 0;
+    for (const Span& s : spans) {
+        if (s.lo < (s.image ? other_end : image_end)) return false;
+        uint64_t& end = s.image ? image_end : other_end;
+        end = std::max(end, s.hi);
+    }
+    return true;
+}
+
 // One pass of the adjoint over device view descriptors dv: vertex records
 // and meshlet normal cones from the current positions, visibility
 // recomputed (clear, cone-only cull: the builder's meshlet bounds do not
@@ -1090,7 +1137,14 @@ int vkgv_diff_graph_capture(vkgv_ctx* ctx, const vkgv_diff_scene* scene, const v
         if (grad_colors) cudaMemsetAsync(reinterpret_cast<void*>(grad_colors), 0, sizeof(float) * nv, s);
         if (grad_texture) cudaMemsetAsync(reinterpret_cast<void*>(grad_texture), 0, sizeof(float) * nt, s);
     }
-    if (passes & VKGV_DIFF_FORWARD) diff_record(ctx, D, g->d_views, view_count, false, s);
+    // A step of both passes is recorded as one: the backward pass recomputes
+    // the visibility anyway, and writes the images while it shades, so
+    // nothing is rasterised or shaded twice (64 views of 512^2 of a
+    // 20,480-triangle sphere: 1,074 -> 752 us a step; 128 views of 256^2 to
+    // 1024^2 of 1.3M triangles: 6.14 -> 3.85 ms).
+    D.A.write_rgb = bwd && (passes & VKGV_DIFF_FORWARD) &&
+                    one_pass_step(*scene, views, view_count, loss, grad_positions, grad_colors, grad_texture);
+    if ((passes & VKGV_DIFF_FORWARD) && !D.A.write_rgb) diff_record(ctx, D, g->d_views, view_count, false, s);
     if (bwd) diff_record(ctx, D, g->d_views, view_count, true, s);
     e = cudaStreamEndCapture(s, &g->graph);
     if (e != cudaSuccess) {

@@ -235,7 +235,9 @@ __device__ __forceinline__ void clip_ab(const float* VP, const float* q, float n
     b = __fadd_rn(__fmaf_rn(-ny, wh, yh), __fmaf_rn(-ny, wl, yl));
 }
 
-// One pixel of the forward image (BACKWARD = false) or of the gradient pass.
+// One pixel of the forward image (BACKWARD = false) or of the gradient pass,
+// which in a captured forward + backward step (A.write_rgb) writes the image
+// too: the same operations in the same order, so the same bits.
 template <bool BACKWARD>
 __device__ __forceinline__ void shade_pixel(const DiffArgs& A, const DeviceView& V, const float* VP, float sn, float cs,
                                             uint32_t p, float& loss_acc) {
@@ -243,6 +245,7 @@ __device__ __forceinline__ void shade_pixel(const DiffArgs& A, const DeviceView&
     const uint32_t lo = (uint32_t)V.depth_id[p];
     float tgt[3] = {0.0f, 0.0f, 0.0f};
     const bool mse = V.diff_target != nullptr;
+    float* out = (!BACKWARD || A.write_rgb) ? V.diff_rgb : nullptr;
     if (BACKWARD && mse) {
         tgt[0] = V.diff_target[3 * p];
         tgt[1] = V.diff_target[3 * p + 1];
@@ -250,7 +253,7 @@ __device__ __forceinline__ void shade_pixel(const DiffArgs& A, const DeviceView&
     }
     if (lo == 0) {
         if (BACKWARD) loss_acc += A.scale * (tgt[0] * tgt[0] + tgt[1] * tgt[1] + tgt[2] * tgt[2]);
-        else if (V.diff_rgb) V.diff_rgb[3 * p] = V.diff_rgb[3 * p + 1] = V.diff_rgb[3 * p + 2] = 0.0f;
+        if (out) out[3 * p] = out[3 * p + 1] = out[3 * p + 2] = 0.0f;
         return;
     }
     const uint4 tvi = A.tri_verts[lo - 1u];
@@ -280,7 +283,7 @@ __device__ __forceinline__ void shade_pixel(const DiffArgs& A, const DeviceView&
     const float sum = fadd(fadd(l[0], l[1]), l[2]);
     if (!(sum != 0.0f)) {  // degenerate: shaded as empty, no gradient
         if (BACKWARD) loss_acc += A.scale * (tgt[0] * tgt[0] + tgt[1] * tgt[1] + tgt[2] * tgt[2]);
-        else if (V.diff_rgb) V.diff_rgb[3 * p] = V.diff_rgb[3 * p + 1] = V.diff_rgb[3 * p + 2] = 0.0f;
+        if (out) out[3 * p] = out[3 * p + 1] = out[3 * p + 2] = 0.0f;
         return;
     }
     float lam[3] = {fdiv(l[0], sum), fdiv(l[1], sum), fdiv(l[2], sum)};
@@ -320,14 +323,12 @@ __device__ __forceinline__ void shade_pixel(const DiffArgs& A, const DeviceView&
         tex[j] = fadd(top, fmul(ay, fsub(bot, top)));
         rgb[j] = fmul(fmul(col[j], A.albedo[j]), tex[j]);
     }
-    if (!BACKWARD) {
-        if (V.diff_rgb) {
-            V.diff_rgb[3 * p] = rgb[0];
-            V.diff_rgb[3 * p + 1] = rgb[1];
-            V.diff_rgb[3 * p + 2] = rgb[2];
-        }
-        return;
+    if (out) {
+        out[3 * p] = rgb[0];
+        out[3 * p + 1] = rgb[1];
+        out[3 * p + 2] = rgb[2];
     }
+    if (!BACKWARD) return;
     // ---- backward
     float g[3], dcol[3], dtex[3];
 #pragma unroll

@@ -105,6 +105,7 @@ struct DiffArgs {
     float uv_scale[2];
     float uv_rotation;
     float scale;
+    uint32_t write_rgb;            // a backward pass also writes the forward image
     float* loss;
     float* grad_positions;
     float* grad_colors;
