@@ -48,7 +48,7 @@ struct vkgv_ctx {
 
     Scratch survivors;  // per view: capacity draw_count
     Scratch rejected;   // per view: capacity draw_count
-    Scratch deferred;   // per view: capacity draw_count
+    Scratch deferred;   // per view: deferred_capacity()
     Scratch reject_samples;  // per view: capacity draw_count (8 B each)
     Scratch diff;       // adjoint: internal raster scene of the differentiable mesh
     Scratch diff_acc;   // adjoint: float4 gradient accumulators (positions, colours, texels)
@@ -211,7 +211,8 @@ int build_views(vkgv_ctx* ctx, const vkgv_scene* scene, const vkgv_view* views, 
     size_t per_view = std::max<size_t>(D, 1) * sizeof(uint32_t);
     rc = ensure_scratch(ctx, ctx->rejected, per_view * n, "rejected lists");
     if (rc) return rc;
-    rc = ensure_scratch(ctx, ctx->deferred, per_view * n, "deferred meshlet lists");
+    const size_t deferred = std::max<size_t>(deferred_capacity(D, ctx->sm_count), 1);
+    rc = ensure_scratch(ctx, ctx->deferred, deferred * sizeof(uint32_t) * n, "deferred meshlet lists");
     if (rc) return rc;
     const bool two_pass = (flags & VKGV_CULL_TWO_PASS) && (flags & VKGV_CULL_OCCLUSION);
     if (two_pass) {
@@ -267,7 +268,7 @@ int build_views(vkgv_ctx* ctx, const vkgv_scene* scene, const vkgv_view* views, 
             d.survivor_capacity = D;
         }
         d.rejected = reinterpret_cast<uint32_t*>(ctx->rejected.ptr) + (size_t)i * std::max<uint32_t>(D, 1);
-        d.deferred = reinterpret_cast<uint32_t*>(ctx->deferred.ptr) + (size_t)i * std::max<uint32_t>(D, 1);
+        d.deferred = reinterpret_cast<uint32_t*>(ctx->deferred.ptr) + (size_t)i * deferred;
         d.reject_samples = two_pass ? reinterpret_cast<unsigned long long*>(ctx->reject_samples.ptr) +
                                           (size_t)i * std::max<uint32_t>(D, 1)
                                     : nullptr;

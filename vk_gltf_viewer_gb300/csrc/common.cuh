@@ -44,7 +44,7 @@ struct DeviceView {
     uint32_t* survivors;        // pass-1 survivors at [0, c[0]), pass-2 at [c[0], c[0]+c[2])
     uint32_t* survivor_count;   // user-visible total (written by the finalize step)
     uint32_t* rejected;         // pass-1 occlusion rejects (scratch)
-    uint32_t* deferred;         // meshlets with clipped or large triangles (scratch, capacity = draws)
+    uint32_t* deferred;         // meshlets with clipped or large triangles (scratch, deferred_capacity())
     // scratch counters: [0] pass-1 survivors, [1] rejects, [2] pass-2 survivors,
     // [3] HiZ tiles done, [4..6] deferred meshlets of raster pass 1 / 2 / explicit list
     uint32_t* counters;

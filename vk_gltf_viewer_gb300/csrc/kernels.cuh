@@ -53,6 +53,8 @@ void launch_clear(const DeviceView* views, uint32_t nviews, uint64_t max_pixels,
                   uint32_t transform_count = 0, float* tdets = nullptr, float* mvps = nullptr);
 void launch_cull(const SceneArgs& S, const DeviceView* views, uint32_t nviews, uint32_t flags, uint32_t pass,
                  uint32_t* status, uint32_t sm_count, cudaStream_t stream);
+// Entries a view's deferred list (DeviceView::deferred) must hold.
+uint32_t deferred_capacity(uint32_t draw_count, uint32_t sm_count);
 // work: two counters that are zero between launches (each launch returns
 // them to zero).
 void launch_raster(const SceneArgs& S, const DeviceView* views, uint32_t nviews, const RasterLists& lists,

@@ -231,17 +231,24 @@ __device__ __noinline__ void setup_and_raster(int32_t X0, int32_t Y0, float Z0, 
     }
 }
 
-__device__ __forceinline__ bool snap(const float4& v, const RasterCtx& c, int32_t& X, int32_t& Y, float& Z) {
-    if (!(v.w > 0.0f)) return false;
-    // one correctly rounded reciprocal of w and three products
+// The 28.8 snap of a vertex with w > 0: one correctly rounded reciprocal of w
+// and three products.  False when it leaves the snapped range.
+__device__ __forceinline__ bool snap_inside(const float4& v, const RasterCtx& c, int32_t& X, int32_t& Y, float& Z) {
     const float rw = __frcp_rn(v.w);
-    const float xd = fmul(v.x, rw), yd = fmul(v.y, rw), zd = fmul(v.z, rw);
+    const float xd = fmul(v.x, rw), yd = fmul(v.y, rw);
     const float xf = fadd(fmul(xd, c.hw), c.hw), yf = fadd(fmul(yd, c.hh), c.hh);
     const float sx = fmul(xf, 256.0f), sy = fmul(yf, 256.0f);
-    if (!(fabsf(sx) < 1073741824.0f) || !(fabsf(sy) < 1073741824.0f)) return false;
     X = __float2int_rn(sx);
     Y = __float2int_rn(sy);
-    Z = zd;
+    Z = fmul(v.z, rw);
+    return fabsf(sx) < 1073741824.0f && fabsf(sy) < 1073741824.0f;
+}
+
+__device__ __forceinline__ bool snap(const float4& v, const RasterCtx& c, int32_t& X, int32_t& Y, float& Z) {
+    int32_t x, y;
+    float z;
+    if (!(v.w > 0.0f) || !snap_inside(v, c, x, y, z)) return false;
+    X = x, Y = y, Z = z;
     return true;
 }
 
@@ -319,10 +326,18 @@ struct ItemHeader {
     uint32_t d;                 // meshlet draw index
     uint32_t v;                 // view (in this launch)
     uint32_t transform;         // node transform index
-    uint8_t vc, tc;             // vertex and triangle counts
-    uint8_t double_sided;       // material flag
-    uint8_t bad;                // an index out of range: reported, skipped
+    uint8_t vc;                 // vertex count
+    uint8_t t0, t1;             // the triangles to draw (none: an index out of range, or no work)
+    uint8_t flags;              // kDoubleSided, kSplit
 };
+constexpr uint8_t kDoubleSided = 1, kSplit = 2;
+constexpr uint32_t kParts = 4;   // 32-triangle rounds of a meshlet
+static_assert(VKGV_MAX_PRIMITIVES <= 32 * kParts, "a meshlet has at most kParts rounds");
+// A deferred meshlet's list entry: the draw index, and for a split item its
+// round and the split flag above it.
+constexpr uint32_t kDeferSplit = 1u << 31;
+constexpr uint32_t kDeferPartShift = VKGV_DRAW_INDEX_BITS;
+constexpr uint32_t kDrawMask = (1u << VKGV_DRAW_INDEX_BITS) - 1u;
 
 struct RasterParams {
     SceneArgs S;
@@ -335,6 +350,8 @@ struct RasterParams {
     uint32_t big_cap;
     uint32_t small_area;
     uint32_t chunk;
+    uint32_t split;           // meshlets at the end of the work list drawn by kParts warps each
+    uint32_t deferred_cap;    // entries a view's deferred list holds
     uint32_t* status;
     uint32_t* work;           // [0] items taken, [1] warps done (zero between launches)
 };
@@ -348,7 +365,7 @@ __device__ __forceinline__ void view_work(const RasterParams& P, const DeviceVie
     first = 0;
     if (SLOW) {
         list = V.deferred;
-        count = min(V.counters[P.lists.deferred_slot], P.S.draw_count);
+        count = min(V.counters[P.lists.deferred_slot], P.deferred_cap);
     } else if (P.lists.pass == 1) {
         list = V.survivors;
         count = min(V.counters[0], V.survivor_capacity);
@@ -365,16 +382,14 @@ __device__ __forceinline__ void view_work(const RasterParams& P, const DeviceVie
 }
 
 // Setup record of one small triangle, shared by the warp while it
-// rasterises all small triangles of a round cooperatively.
-struct TriRec {
-    int32_t x[3], y[3];   // oriented (positive area) snapped vertices, 28.8
+// rasterises all small triangles of a round cooperatively: 32 bytes, two
+// 16-byte words.  Vertices are relative to the corner of the clamped bbox
+// (a small triangle's extent keeps them inside int16).
+struct __align__(16) TriRec {
+    uint32_t v[3];        // oriented (positive area) snapped vertices, 28.8: x | y << 16
+    uint32_t bits;        // triangle (7) | edge biases (3) | bbox width (7) | ceil(4096 / width) (13)
     float z0, pa, pb;     // depth plane
-    float inv_bw;         // 1 / bbox width (exact floor division for bw <= 64)
-    uint32_t id;
-    uint16_t bx0, by0;    // clamped bbox origin (pixels)
-    uint8_t bw, bh;       // clamped bbox extent (pixels, <= 64)
-    uint8_t bias;         // bit k: edge k excludes its samples (not top-left)
-    uint8_t _pad;
+    uint32_t origin;      // clamped bbox origin in pixels: x | y << 16
 };
 
 constexpr uint8_t kFlagGuard = 1u << 6;
@@ -387,6 +402,16 @@ enum TriKind : int { kDrop = 0, kFast = 1, kSlowClip = 2, kSlowSetup = 3 };
 
 #ifndef VKGV_RASTER_WARPS_PER_SM
 #define VKGV_RASTER_WARPS_PER_SM 28
+#endif
+
+// Meshlets at the end of a launch's work list that are split (see k_raster),
+// per SM.  A quarter of the resident warps: 443 meshlets of a 1280x720 view
+// 44 -> 20 us (they had one warp each on a chip of 4,256); the 1080p torus grid's
+// frame 342 -> 326 us (the last heavy meshlets, up to 30 us each, and pass 2's
+// few hundred).  None: 344 us; 14: 327; 28: 329; 56: 341 (every split meshlet
+// transforms its vertices four times).
+#ifndef VKGV_RASTER_SPLIT_PER_SM
+#define VKGV_RASTER_SPLIT_PER_SM 7
 #endif
 
 // Small triangles whose clamped bbox has at most this many pixels are
@@ -402,7 +427,8 @@ constexpr uint32_t kLaneArea = VKGV_RASTER_LANE_AREA;
 constexpr uint32_t kQueueArea = VKGV_RASTER_QUEUE_AREA;
 
 struct TriClass {
-    int4 q0, q1, q2;  // snapped vertex records {X, Y, Z bits, flags}
+    int2 q0, q1, q2;  // snapped vertices
+    int2 f0, f1, f2;  // {depth bits, flags}
 };
 
 // Sorts one meshlet triangle into drop / fast / slow-clip / slow-setup.  The
@@ -412,17 +438,17 @@ struct TriClass {
 // non-zero area, a pixel centre in its bbox, bbox within small_area pixels
 // and edge values within int32.
 template <bool SLOW>
-__device__ __forceinline__ int classify(uint32_t i0, uint32_t i1, uint32_t i2, uint32_t vc, const int4* svtx,
-                                        const float4* clip, bool double_sided, float tdet, const RasterCtx& c,
+__device__ __forceinline__ int classify(uint32_t i0, uint32_t i1, uint32_t i2, uint32_t vc, const int2* sxy,
+                                        const int2* szf, const float4* clip, bool double_sided, float tdet, const RasterCtx& c,
                                         uint32_t d, TriClass& k) {
     if (i0 >= vc || i1 >= vc || i2 >= vc) {
         if (!SLOW) report(c.status, kStatusBadIndex, d);
         return kDrop;
     }
-    k.q0 = svtx[i0];
-    k.q1 = svtx[i1];
-    k.q2 = svtx[i2];
-    const uint32_t f0 = (uint32_t)k.q0.w, f1 = (uint32_t)k.q1.w, f2 = (uint32_t)k.q2.w;
+    k.q0 = sxy[i0], k.f0 = szf[i0];
+    k.q1 = sxy[i1], k.f1 = szf[i1];
+    k.q2 = sxy[i2], k.f2 = szf[i2];
+    const uint32_t f0 = (uint32_t)k.f0.y, f1 = (uint32_t)k.f1.y, f2 = (uint32_t)k.f2.y;
     auto backfacing = [&]() {
         if (double_sided) return false;
         const float4 a = clip[i0], b = clip[i1], cc = clip[i2];
@@ -432,7 +458,7 @@ __device__ __forceinline__ int classify(uint32_t i0, uint32_t i1, uint32_t i2, u
     if (f0 & f1 & f2 & 63) return kDrop;  // outcode reject
     if ((f0 | f1 | f2) & (OC_ZLO | OC_ZHI | kFlagGuard)) return backfacing() ? kDrop : kSlowClip;
     if (!(f0 & f1 & f2 & kFlagSnapped)) return kDrop;
-    const int4 &q0 = k.q0, &q1 = k.q1, &q2 = k.q2;
+    const int2 &q0 = k.q0, &q1 = k.q1, &q2 = k.q2;
     const int32_t minx = min(q0.x, min(q1.x, q2.x)), maxx = max(q0.x, max(q1.x, q2.x));
     const int32_t miny = min(q0.y, min(q1.y, q2.y)), maxy = max(q0.y, max(q1.y, q2.y));
     const int32_t qx0 = max((minx - 128 + 255) >> 8, 0), qx1 = min((maxx - 128) >> 8, (int32_t)c.w - 1);
@@ -453,17 +479,13 @@ __device__ __forceinline__ int classify(uint32_t i0, uint32_t i1, uint32_t i2, u
 // (visbuffer.mesh.glsl:86-101), the zero-area test and the size limits.
 // The tests only filter, so their order does not change what is drawn; the
 // cheap ones run here on every triangle, the others only on the candidates.
-__device__ __forceinline__ int prefilter(uint32_t i0, uint32_t i1, uint32_t i2, uint32_t vc, const int4* svtx,
-                                         const RasterCtx& c, uint32_t d) {
-    if (i0 >= vc || i1 >= vc || i2 >= vc) {
-        report(c.status, kStatusBadIndex, d);
-        return 0;
-    }
-    const int4 q0 = svtx[i0], q1 = svtx[i1], q2 = svtx[i2];
-    const uint32_t f0 = (uint32_t)q0.w, f1 = (uint32_t)q1.w, f2 = (uint32_t)q2.w;
+__device__ __forceinline__ int prefilter(uint32_t i0, uint32_t i1, uint32_t i2, const int2* sxy, const int2* szf,
+                                         const RasterCtx& c) {
+    const uint32_t f0 = (uint32_t)szf[i0].y, f1 = (uint32_t)szf[i1].y, f2 = (uint32_t)szf[i2].y;
     if (f0 & f1 & f2 & 63) return 0;  // outcode reject
     if ((f0 | f1 | f2) & (OC_ZLO | OC_ZHI | kFlagGuard)) return 2;
     if (!(f0 & f1 & f2 & kFlagSnapped)) return 0;
+    const int2 q0 = sxy[i0], q1 = sxy[i1], q2 = sxy[i2];
     const int32_t minx = min(q0.x, min(q1.x, q2.x)), maxx = max(q0.x, max(q1.x, q2.x));
     const int32_t miny = min(q0.y, min(q1.y, q2.y)), maxy = max(q0.y, max(q1.y, q2.y));
     const int32_t qx0 = max((minx - 128 + 255) >> 8, 0), qx1 = min((maxx - 128) >> 8, (int32_t)c.w - 1);
@@ -471,21 +493,40 @@ __device__ __forceinline__ int prefilter(uint32_t i0, uint32_t i1, uint32_t i2, 
     return (qx0 > qx1 || qy0 > qy1) ? 0 : 1;
 }
 
-// One sample of a small triangle: int32 edge functions (the extent bound of
-// kFast keeps them exact), top-left bias, plane depth clamped to [0, 1].
-__device__ __forceinline__ void small_sample(const int32_t* x, const int32_t* y, uint32_t bias, float z0, float pa,
-                                             float pb, int32_t px, int32_t py, unsigned long long lo,
-                                             const RasterCtx& c) {
-    const int32_t sx = px * 256 + 128, sy = py * 256 + 128;
-    const int32_t e0 = (x[1] - x[0]) * (sy - y[0]) - (y[1] - y[0]) * (sx - x[0]);
-    const int32_t e1 = (x[2] - x[1]) * (sy - y[1]) - (y[2] - y[1]) * (sx - x[1]);
-    const int32_t e2 = (x[0] - x[2]) * (sy - y[2]) - (y[0] - y[2]) * (sx - x[2]);
-    if (e0 >= (int32_t)(bias & 1u) && e1 >= (int32_t)((bias >> 1) & 1u) && e2 >= (int32_t)((bias >> 2) & 1u)) {
-        float z = __fmaf_rn(pa, __int2float_rn(sx - x[0]), __fmaf_rn(pb, __int2float_rn(sy - y[0]), z0));
-        if (!(z > 0.0f)) z = 0.0f;
-        if (z > 1.0f) z = 1.0f;
-        plot(c.depth + (size_t)py * c.w + px, ((unsigned long long)__float_as_uint(z) << 32) | lo);
-    }
+// The same for a meshlet whose vertices all lie inside the view volume: no
+// flag is set and the view clamps nothing (the snapped coordinates are in
+// [0, 256 w] x [0, 256 h]), which leaves the empty-box test.  With u = x - 128
+// the pixel centres are the multiples of 256, and [min u, max u] holds none
+// exactly when min u - 1 and max u share their quotient by 256.
+__device__ __forceinline__ bool covers_centre(int2 q0, int2 q1, int2 q2) {
+    const uint32_t x = (uint32_t)(min(q0.x, min(q1.x, q2.x)) - 129) ^ (uint32_t)(max(q0.x, max(q1.x, q2.x)) - 128);
+    const uint32_t y = (uint32_t)(min(q0.y, min(q1.y, q2.y)) - 129) ^ (uint32_t)(max(q0.y, max(q1.y, q2.y)) - 128);
+    return x > 255u && y > 255u;
+}
+
+// A small triangle's edge functions and depth plane at a sample, relative to
+// its bbox corner: int32 values (the extent bound of a small triangle keeps
+// them exact) with the top-left biases subtracted, so that the sample is
+// covered when no sign bit is set.
+struct SmallEdges {
+    int32_t e0, e1, e2;     // at the current sample
+    int32_t ax, ay, bx, by, cx, cy;  // edge vectors
+    float fx, fy;           // sample - vertex 0
+};
+
+__device__ __forceinline__ void edges_at(SmallEdges& s, int32_t x0, int32_t y0, int32_t x1, int32_t y1, int32_t x2,
+                                         int32_t y2, uint32_t bias, int32_t sx, int32_t sy) {
+    s.ax = x1 - x0, s.ay = y1 - y0, s.bx = x2 - x1, s.by = y2 - y1, s.cx = x0 - x2, s.cy = y0 - y2;
+    s.e0 = s.ax * (sy - y0) - s.ay * (sx - x0) - (int32_t)(bias & 1u);
+    s.e1 = s.bx * (sy - y1) - s.by * (sx - x1) - (int32_t)((bias >> 1) & 1u);
+    s.e2 = s.cx * (sy - y2) - s.cy * (sx - x2) - (int32_t)((bias >> 2) & 1u);
+    s.fx = __int2float_rn(sx - x0), s.fy = __int2float_rn(sy - y0);
+}
+
+// Depth of a covered sample, clamped to [0, 1] (NaN and -0 to +0), over id + 1.
+__device__ __forceinline__ unsigned long long fragment(float pa, float pb, float z0, float fx, float fy, uint32_t id) {
+    const float z = __saturatef(__fmaf_rn(pa, fx, __fmaf_rn(pb, fy, z0)));
+    return ((unsigned long long)__float_as_uint(z) << 32) | (unsigned long long)(id + 1u);
 }
 
 // Second stage of the fast instance: up to 32 compacted candidates, one
@@ -495,89 +536,92 @@ __device__ __forceinline__ void small_sample(const int32_t* x, const int32_t* y,
 // the slow instance (the return value); the rest are set up and
 // rasterised.  A triangle whose
 // clamped bbox has at most kLaneArea pixels is rasterised by its own lane;
-// the larger ones are spread over the warp by an inclusive scan of their
-// bbox areas.
-__device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, const int4* svtx, const float4* clip,
+// the larger ones are spread over the warp by a scan of their bbox areas.
+// xyw holds each vertex's clip x, y, w and snapped depth.
+__device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, const int2* sxy, const float4* xyw,
                                              bool double_sided, float tdet, uint32_t d, const RasterCtx& c,
-                                             TriRec* recs, uint32_t* ends, int lane) {
+                                             TriRec* recs, uint32_t* starts, int lane) {
     uint32_t coop_area = 0;
     bool slow = false;
-    int4 q0, q1, q2;
-    int32_t A = 0;  // the area of a live (small) triangle fits int32
-    int32_t px0 = 0, px1 = 0, py0 = 0, py1 = 0;
-    bool live = false;
+    TriRec rec;
     if (ct != 0xffffffffu) {
         const uint32_t i0 = sidx8[3 * ct], i1 = sidx8[3 * ct + 1], i2 = sidx8[3 * ct + 2];
-        q0 = svtx[i0], q1 = svtx[i1], q2 = svtx[i2];
+        const int2 q0 = sxy[i0], q1 = sxy[i1], q2 = sxy[i2];
+        const float4 k0 = xyw[i0], k1 = xyw[i1], k2 = xyw[i2];
         bool back = false;
         if (!double_sided) {
-            const float4 a = clip[i0], b = clip[i1], cc = clip[i2];
-            const float det = det3(a.x, a.y, a.w, b.x, b.y, b.w, cc.x, cc.y, cc.w);
+            const float det = det3(k0.x, k0.y, k0.z, k1.x, k1.y, k1.z, k2.x, k2.y, k2.z);
             back = tdet < 0.0f ? det < 0.0f : det > 0.0f;
         }
-        if (!back) {
-            const int32_t minx = min(q0.x, min(q1.x, q2.x)), maxx = max(q0.x, max(q1.x, q2.x));
-            const int32_t miny = min(q0.y, min(q1.y, q2.y)), maxy = max(q0.y, max(q1.y, q2.y));
-            if (maxx - minx < kSmallExtent && maxy - miny < kSmallExtent) {
-                // edge values of such a triangle stay inside int32
-                A = (q1.x - q0.x) * (q2.y - q0.y) - (q1.y - q0.y) * (q2.x - q0.x);
-                px0 = max((minx - 128 + 255) >> 8, 0), px1 = min((maxx - 128) >> 8, (int32_t)c.w - 1);
-                py0 = max((miny - 128 + 255) >> 8, 0), py1 = min((maxy - 128) >> 8, (int32_t)c.h - 1);
-                if (A != 0) {
-                    live = (uint32_t)((px1 - px0 + 1) * (py1 - py0 + 1)) <= c.small_area;
-                    slow = !live;
+        const int32_t minx = min(q0.x, min(q1.x, q2.x)), maxx = max(q0.x, max(q1.x, q2.x));
+        const int32_t miny = min(q0.y, min(q1.y, q2.y)), maxy = max(q0.y, max(q1.y, q2.y));
+        const bool fits = maxx - minx < kSmallExtent && maxy - miny < kSmallExtent;
+        // edge values of a triangle of that extent stay inside int32 (the
+        // area of a larger one wraps and is not used)
+        const int32_t A = (int32_t)((uint32_t)(q1.x - q0.x) * (uint32_t)(q2.y - q0.y) -
+                                    (uint32_t)(q1.y - q0.y) * (uint32_t)(q2.x - q0.x));
+        const int32_t px0 = max((minx - 128 + 255) >> 8, 0), px1 = min((maxx - 128) >> 8, (int32_t)c.w - 1);
+        const int32_t py0 = max((miny - 128 + 255) >> 8, 0), py1 = min((maxy - 128) >> 8, (int32_t)c.h - 1);
+        const uint32_t bw = (uint32_t)(px1 - px0 + 1), bh = (uint32_t)(py1 - py0 + 1);
+        const bool live = !back && fits && A != 0 && bw * bh <= c.small_area;
+        if (!back && !live) {
+            const int64_t A64 = (int64_t)(q1.x - q0.x) * (q2.y - q0.y) - (int64_t)(q1.y - q0.y) * (q2.x - q0.x);
+            slow = A64 != 0;
+        }
+        if (live) {
+            const bool flip = A < 0;  // orient to positive area
+            const int32_t ox = px0 << 8, oy = py0 << 8;
+            const int32_t x0 = q0.x - ox, y0 = q0.y - oy;
+            const int32_t x1 = (flip ? q2.x : q1.x) - ox, y1 = (flip ? q2.y : q1.y) - oy;
+            const int32_t x2 = (flip ? q1.x : q2.x) - ox, y2 = (flip ? q1.y : q2.y) - oy;
+            const float z0 = k0.w, z1 = flip ? k2.w : k1.w, z2 = flip ? k1.w : k2.w;
+            const int32_t ax = x1 - x0, ay = y1 - y0, bx = x2 - x1, by = y2 - y1, cx = x0 - x2, cy = y0 - y2;
+            // an edge that is not top-left excludes its samples
+            const uint32_t bias = ((ay < 0 || (ay == 0 && ax > 0)) ? 0u : 1u) | ((by < 0 || (by == 0 && bx > 0)) ? 0u : 2u) |
+                                  ((cy < 0 || (cy == 0 && cx > 0)) ? 0u : 4u);
+            const float dx1 = __int2float_rn(ax), dy1 = __int2float_rn(ay);
+            const float dx2 = __int2float_rn(-cx), dy2 = __int2float_rn(-cy);
+            const float dz1 = fsub(z1, z0), dz2 = fsub(z2, z0);
+            const float ra = __frcp_rn(__int2float_rn(flip ? -A : A));
+            const float pa = fmul(fsub(fmul(dz1, dy2), fmul(dz2, dy1)), ra);
+            const float pb = fmul(fsub(fmul(dz2, dx1), fmul(dz1, dx2)), ra);
+            if (bw * bh <= kLaneArea) {
+                SmallEdges e;
+                edges_at(e, x0, y0, x1, y1, x2, y2, bias, 128, 128);
+                const uint32_t id = (d << 7) | ct;
+                unsigned long long* row = c.depth + (size_t)(uint32_t)py0 * c.w + (uint32_t)px0;
+                for (uint32_t ly = bh;;) {
+                    int32_t r0 = e.e0, r1 = e.e1, r2 = e.e2;
+                    float fx = e.fx;
+                    unsigned long long* p = row;
+                    for (uint32_t lx = bw;;) {
+                        if ((r0 | r1 | r2) >= 0) plot(p, fragment(pa, pb, z0, fx, e.fy, id));
+                        if (--lx == 0) break;
+                        r0 -= e.ay << 8, r1 -= e.by << 8, r2 -= e.cy << 8;
+                        fx = fadd(fx, 256.0f);  // whole numbers below 2^24: exact
+                        ++p;
+                    }
+                    if (--ly == 0) break;
+                    e.e0 += e.ax << 8, e.e1 += e.bx << 8, e.e2 += e.cx << 8;
+                    e.fy = fadd(e.fy, 256.0f);
+                    row += c.w;
                 }
             } else {
-                const int64_t A64 = (int64_t)(q1.x - q0.x) * (q2.y - q0.y) - (int64_t)(q1.y - q0.y) * (q2.x - q0.x);
-                slow = A64 != 0;
+                rec.v[0] = ((uint32_t)x0 & 0xFFFFu) | ((uint32_t)y0 << 16);
+                rec.v[1] = ((uint32_t)x1 & 0xFFFFu) | ((uint32_t)y1 << 16);
+                rec.v[2] = ((uint32_t)x2 & 0xFFFFu) | ((uint32_t)y2 << 16);
+                // ceil(4096 / bw): 4096 times the correctly rounded 1 / bw
+                // rounded up (whole only for the powers of two, exact there)
+                const uint32_t inv = __float2uint_ru(fmul(4096.0f, __frcp_rn((float)bw)));
+                rec.bits = ct | (bias << 7) | (bw << 10) | (inv << 17);
+                rec.z0 = z0, rec.pa = pa, rec.pb = pb;
+                rec.origin = (uint32_t)px0 | ((uint32_t)py0 << 16);
+                coop_area = bw * bh;
             }
         }
     }
-    if (live) {
-        int32_t x[3] = {q0.x, q1.x, q2.x}, y[3] = {q0.y, q1.y, q2.y};
-        float z0 = __int_as_float(q0.z), z1 = __int_as_float(q1.z), z2 = __int_as_float(q2.z);
-        if (A < 0) {  // orient to positive area
-            x[1] = q2.x, y[1] = q2.y, x[2] = q1.x, y[2] = q1.y;
-            z1 = __int_as_float(q2.z), z2 = __int_as_float(q1.z);
-        }
-        const int32_t Ap = A < 0 ? -A : A;
-        const uint32_t bw = (uint32_t)(px1 - px0 + 1), bh = (uint32_t)(py1 - py0 + 1);
-        uint32_t bias = 0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const int32_t dx = x[(k + 1) % 3] - x[k], dy = y[(k + 1) % 3] - y[k];
-            if (!(dy < 0 || (dy == 0 && dx > 0))) bias |= 1u << k;
-        }
-        const float dx1 = __int2float_rn(x[1] - x[0]), dy1 = __int2float_rn(y[1] - y[0]);
-        const float dx2 = __int2float_rn(x[2] - x[0]), dy2 = __int2float_rn(y[2] - y[0]);
-        const float af = __int2float_rn(Ap);
-        const float dz1 = fsub(z1, z0), dz2 = fsub(z2, z0);
-        const float ra = __frcp_rn(af);
-        const float pa = fmul(fsub(fmul(dz1, dy2), fmul(dz2, dy1)), ra);
-        const float pb = fmul(fsub(fmul(dz2, dx1), fmul(dz1, dx2)), ra);
-        const uint32_t id = (d << 7) | ct;
-        if (bw * bh <= kLaneArea) {
-            const unsigned long long lo = (unsigned long long)id + 1ull;
-            for (uint32_t ly = 0; ly < bh; ++ly)
-                for (uint32_t lx = 0; lx < bw; ++lx)
-                    small_sample(x, y, bias, z0, pa, pb, px0 + (int32_t)lx, py0 + (int32_t)ly, lo, c);
-        } else {
-            TriRec& r = recs[lane];
-            r.x[0] = x[0], r.x[1] = x[1], r.x[2] = x[2];
-            r.y[0] = y[0], r.y[1] = y[1], r.y[2] = y[2];
-            r.z0 = z0;
-            r.pa = pa;
-            r.pb = pb;
-            r.inv_bw = 1.0f / (float)bw;
-            r.id = id;
-            r.bx0 = (uint16_t)px0;
-            r.by0 = (uint16_t)py0;
-            r.bw = (uint8_t)bw;
-            r.bh = (uint8_t)bh;
-            r.bias = (uint8_t)bias;
-            coop_area = bw * bh;
-        }
-    }
+    unsigned coop = __ballot_sync(0xffffffffu, coop_area != 0);
+    if (coop == 0) return slow;
     // Triangles whose bbox exceeds kQueueArea pixels go to the
     // binned-rectangle queue (one rectangle each), drained by k_raster_big
     // with a warp per rectangle: a meshlet of larger triangles then no
@@ -592,14 +636,17 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
         if (coop_area > kQueueArea) {
             const uint32_t slot = base + (uint32_t)__popc(mm & ((1u << lane) - 1u));
             if (slot < c.big_cap) {
-                const TriRec& r = recs[lane];
+                const uint32_t px0 = rec.origin & 0xFFFFu, py0 = rec.origin >> 16, bw = (rec.bits >> 10) & 127u;
                 BigTri t;
-                t.x[0] = r.x[0], t.x[1] = r.x[1], t.x[2] = r.x[2];
-                t.y[0] = r.y[0], t.y[1] = r.y[1], t.y[2] = r.y[2];
-                t.z0 = r.z0, t.pa = r.pa, t.pb = r.pb;
-                t.id = r.id;
-                t.px0 = r.bx0, t.py0 = r.by0;
-                t.px1 = (uint16_t)(r.bx0 + r.bw - 1), t.py1 = (uint16_t)(r.by0 + r.bh - 1);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    t.x[k] = (int32_t)(int16_t)(rec.v[k] & 0xFFFFu) + (int32_t)(px0 << 8);
+                    t.y[k] = ((int32_t)rec.v[k] >> 16) + (int32_t)(py0 << 8);
+                }
+                t.z0 = rec.z0, t.pa = rec.pa, t.pb = rec.pb;
+                t.id = (d << 7) | (rec.bits & 127u);
+                t.px0 = (uint16_t)px0, t.py0 = (uint16_t)py0;
+                t.px1 = (uint16_t)(px0 + bw - 1u), t.py1 = (uint16_t)(py0 + coop_area / bw - 1u);
                 t.view = c.view;
                 t._pad = 0;
                 c.big[slot] = t;
@@ -608,31 +655,46 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
                 report(c.status, kStatusQueueOverflow, slot);
             }
         }
+        coop = __ballot_sync(0xffffffffu, coop_area != 0);
+        if (coop == 0) return slow;
     }
-    if (__ballot_sync(0xffffffffu, coop_area != 0) == 0) return slow;
-    // Warp-cooperative raster: an inclusive scan of the bbox areas spreads
-    // the pixels of the larger small triangles evenly over the lanes.
+    // Warp-cooperative raster: the records compacted in lane order and a scan
+    // of their bbox areas spread the pixels evenly over the lanes.  A lane
+    // finds its pixel's record by counting the records that start at or before
+    // it: those before this step's 32 pixels by a ballot, the others in a mask
+    // of the start positions.
     uint32_t incl = coop_area;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += v;
     }
-    ends[lane] = incl;
     const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    const uint32_t start = coop_area ? incl - coop_area : 0xffffffffu;
+    if (coop_area) {
+        const uint32_t at = (uint32_t)__popc(coop & ((1u << lane) - 1u));
+        recs[at] = rec;
+        starts[at] = start;
+    }
     __syncwarp();
-    for (uint32_t p = lane; p < total; p += 32) {
-        // smallest j with ends[j] > p
-        uint32_t j = 0;
-#pragma unroll
-        for (uint32_t step = 16; step > 0; step >>= 1)
-            if (ends[j + step - 1] <= p) j += step;
-        const TriRec& r = recs[j];
-        const uint32_t local = p - (ends[j] - (uint32_t)r.bw * r.bh);
-        const uint32_t ly = (uint32_t)(((float)local + 0.5f) * r.inv_bw);
-        const uint32_t lx = local - ly * r.bw;
-        small_sample(r.x, r.y, r.bias, r.z0, r.pa, r.pb, (int32_t)(r.bx0 + lx), (int32_t)(r.by0 + ly),
-                     (unsigned long long)r.id + 1ull, c);
+    for (uint32_t p0 = 0; p0 < total; p0 += 32) {
+        const uint32_t before = (uint32_t)__popc(__ballot_sync(0xffffffffu, start < p0));
+        const uint32_t mine = start - p0 < 32u ? 1u << (start - p0) : 0u;
+        const uint32_t begins = __reduce_or_sync(0xffffffffu, mine);
+        const uint32_t p = p0 + (uint32_t)lane;
+        if (p < total) {
+            const uint32_t j = before + (uint32_t)__popc(begins & (0xffffffffu >> (31 - lane))) - 1u;
+            const TriRec r = recs[j];
+            const uint32_t local = p - starts[j], bw = (r.bits >> 10) & 127u;
+            const uint32_t ly = (local * (r.bits >> 17)) >> 12, lx = local - ly * bw;
+            SmallEdges e;
+            edges_at(e, (int32_t)(int16_t)(r.v[0] & 0xFFFFu), (int32_t)r.v[0] >> 16, (int32_t)(int16_t)(r.v[1] & 0xFFFFu),
+                     (int32_t)r.v[1] >> 16, (int32_t)(int16_t)(r.v[2] & 0xFFFFu), (int32_t)r.v[2] >> 16,
+                     (r.bits >> 7) & 7u, (int32_t)(lx << 8) + 128, (int32_t)(ly << 8) + 128);
+            if ((e.e0 | e.e1 | e.e2) >= 0)
+                plot(c.depth + (size_t)((r.origin >> 16) + ly) * c.w + (r.origin & 0xFFFFu) + lx,
+                     fragment(r.pa, r.pb, r.z0, e.fx, e.fy, (d << 7) | (r.bits & 127u)));
+        }
     }
     __syncwarp();
     return slow;
@@ -647,15 +709,19 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
 template <int WARPS, bool SLOW>
 __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER_SM) / WARPS) k_raster(RasterParams P) {
     pdl_begin();
+    // per vertex: clip {x, y, z, w} (slow instance) or clip {x, y, w} and the
+    // snapped depth (fast instance); the snapped {X, Y} (28.8); {depth bits,
+    // flags}, which the fast instance reads only for a meshlet that is not
+    // entirely inside the view volume
     __shared__ float4 s_clip[WARPS][64];
-    // per vertex: {X, Y (28.8), Z bits, flags} read with one 16-byte load
-    __shared__ int4 s_vtx[WARPS][64];
+    __shared__ int2 s_xy[WARPS][64];
+    __shared__ int2 s_zf[WARPS][64];
     // the meshlet's triangle-index bytes (<= 126 triangles)
     __shared__ uint32_t s_idx[WARPS][96];
     __shared__ TriRec s_tri[WARPS][32];
-    // ring of compacted candidate triangle indices (fast instance)
-    __shared__ uint8_t s_ring[WARPS][64];
-    __shared__ uint32_t s_end[WARPS][32];
+    // the compacted candidate triangle indices (fast instance)
+    __shared__ uint8_t s_ring[WARPS][128];
+    __shared__ uint32_t s_start[WARPS][32];
     __shared__ float s_mvp[WARPS][16];
     __shared__ float s_tdet[WARPS];
     __shared__ float s_vp[WARPS][16];
@@ -691,15 +757,20 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
         }
     }
     __syncthreads();
-    const uint32_t total = s_pre[nv];
+    // The last `split` meshlets of the list are drawn by kParts warps each, one
+    // 32-triangle round a warp: a launch of few meshlets then fills the chip
+    // (and the longest of them takes one round, not four), and at the end of
+    // a long one the last warps are not left alone with whole heavy meshlets.
+    const uint32_t total = s_pre[nv] + (kParts - 1) * min(s_pre[nv], P.split);
     const uint32_t slot = P.lists.deferred_slot;
-    const uint32_t defer_cap = P.S.draw_count;
+    const uint32_t defer_cap = P.deferred_cap;
     float4* clip = s_clip[warp];
-    int4* svtx = s_vtx[warp];
+    int2* sxy = s_xy[warp];
+    int2* szf = s_zf[warp];
     uint32_t* sidx = s_idx[warp];
     const uint8_t* sidx8 = reinterpret_cast<const uint8_t*>(sidx);
     TriRec* recs = s_tri[warp];
-    uint32_t* ends = s_end[warp];
+    uint32_t* starts = s_start[warp];
     // Warps take runs of `grab` consecutive work items from one counter, so
     // views are drawn roughly in order (their depth buffers stay in L2) and
     // no warp idles while work is left.
@@ -736,12 +807,19 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
         if (lane == 0) next = atomicAdd(P.work, grab);
         const uint32_t stop = min(base + grab, total);
         {
-            const uint32_t g = base + (uint32_t)lane;
+            uint32_t g = base + (uint32_t)lane;
             ItemHeader h;
             h.d = 0xffffffffu;
             h.v = 0;
-            h.bad = 1;
+            h.t0 = h.t1 = 0;
             if (g < stop) {
+                const uint32_t whole = s_pre[nv] - min(s_pre[nv], P.split);
+                bool split = g >= whole;
+                uint32_t part = 0;
+                if (split) {
+                    part = (g - whole) % kParts;
+                    g = whole + (g - whole) / kParts;
+                }
                 // the view holding g: the last v with s_pre[v] <= g
                 uint32_t v = 0, hi = nv;
                 while (v + 1 < hi) {
@@ -752,9 +830,18 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
                 const uint32_t* list;
                 uint32_t n, first;
                 view_work<SLOW>(P, P.views[v], list, n, first);
-                const uint32_t d = list[first + (g - s_pre[v])];
+                uint32_t d = list[first + (g - s_pre[v])];
+                bool skip = false;  // a deferred round that another part of this entry draws
+                if (SLOW && (d & kDeferSplit)) {
+                    const uint32_t own = (d >> kDeferPartShift) % kParts;
+                    skip = split && part != own;
+                    split = true;
+                    part = own;
+                    d &= kDrawMask;
+                }
                 h.v = v;
                 h.d = d;
+                bool bad = true;
                 if (d < P.S.draw_count) {
                     const vkgv_meshlet_draw dr = P.S.draws[d];
                     const vkgv_primitive* prim = &P.S.prims[dr.primitive_index];
@@ -768,12 +855,17 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
                             h.verts = reinterpret_cast<const vkgv_vertex*>(prim->vertex_buffer);
                             h.transform = dr.transform_index;
                             h.vc = (uint8_t)vc;
-                            h.tc = (uint8_t)tc;
-                            h.double_sided = P.S.mats[prim->material_index].double_sided != 0 ? 1 : 0;
-                            h.bad = 0;
+                            if (!skip) {
+                                h.t0 = (uint8_t)(split ? 32u * part : 0u);
+                                h.t1 = (uint8_t)(split ? min(tc, 32u * part + 32u) : tc);
+                            }
+                            h.flags = (uint8_t)((P.S.mats[prim->material_index].double_sided != 0 ? kDoubleSided : 0) |
+                                                (split ? kSplit : 0));
+                            bad = false;
                         }
                     }
                 }
+                if (bad) report(P.status, kStatusBadIndex, d);
             }
             __syncwarp();  // every lane is done with the previous run's headers
             hdr[lane] = h;
@@ -781,11 +873,8 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
         __syncwarp();
         for (uint32_t k = 0; k < stop - base; ++k) {
             const ItemHeader& H = hdr[k];
+            if (H.t0 >= H.t1) continue;
             const uint32_t v = H.v, d = H.d;
-            if (H.bad) {
-                if (lane == 0) report(P.status, kStatusBadIndex, d);
-                continue;
-            }
             if (v != cur_v) {
                 cur_v = v;
                 cur_t = 0xffffffffu;
@@ -803,11 +892,11 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
                 __syncwarp();
             }
             const DeviceView& V = *Vp;
-            const uint32_t vc = H.vc, tc = H.tc;
+            const uint32_t vc = H.vc, tc = H.t1;
             const uint32_t* vidx = H.vidx;
             const uint8_t* tri = H.tri;
             const vkgv_vertex* verts = H.verts;
-            const bool double_sided = H.double_sided != 0;
+            const bool double_sided = (H.flags & kDoubleSided) != 0;
             const uint32_t transform_index = H.transform;
             // mvp = VP * M, one element per lane (lanes 0-15); lane 16 takes the
             // sign source determinant(M) of visbuffer.mesh.glsl:71.
@@ -863,20 +952,36 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
                 xy1 = __ldg(reinterpret_cast<const float2*>(vx1->position));
                 zz1 = __ldg(&vx1->position[2]);
             }
-            auto vertex = [&](uint32_t k, float px, float py, float pz) {
-                float r[4];
-                m4v(mvp, px, py, pz, 1.0f, r);
-                const float4 cv = make_float4(r[0], r[1], r[2], r[3]);
-                clip[k] = cv;
+            float4 cv[2];
+            m4v(mvp, xy0.x, xy0.y, zz0, 1.0f, &cv[0].x);
+            m4v(mvp, xy1.x, xy1.y, zz1, 1.0f, &cv[1].x);
+            // Inside the view volume no outcode, guard or snap-range test can
+            // fire: a meshlet with all vertices inside skips them here and in
+            // the pre-filter (issue-bound: 256 views of 128^2 1,731 -> 1,474 us
+            // a frame, the 256-view torus grid 37.0 -> 32.2 ms, with the
+            // pre-filter on 8-byte vertices and the relative edge setup).
+            auto inside = [](const float4& q) {
+                return fabsf(q.x) <= q.w && fabsf(q.y) <= q.w && q.z >= 0.0f && q.z <= q.w && q.w > 0.0f;
+            };
+            const bool plain = !SLOW && __all_sync(0xffffffffu, (!h0 || inside(cv[0])) && (!h1 || inside(cv[1])));
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                if (!(q ? h1 : h0)) continue;
+                const uint32_t k = (uint32_t)lane + 32u * q;
+                const float4 v = cv[q];
                 int32_t X = 0, Y = 0;
                 float Z = 0.0f;
-                uint32_t fl = (uint32_t)outcode(cv);
-                if (outside_guard(cv)) fl |= kFlagGuard;
-                if (snap(cv, c, X, Y, Z)) fl |= kFlagSnapped;
-                svtx[k] = make_int4(X, Y, __float_as_int(Z), (int)fl);
-            };
-            if (h0) vertex(lane, xy0.x, xy0.y, zz0);
-            if (h1) vertex(lane + 32, xy1.x, xy1.y, zz1);
+                if (plain) {
+                    snap_inside(v, c, X, Y, Z);
+                } else {
+                    uint32_t fl = (uint32_t)outcode(v);
+                    if (outside_guard(v)) fl |= kFlagGuard;
+                    if (snap(v, c, X, Y, Z)) fl |= kFlagSnapped;
+                    szf[k] = make_int2(__float_as_int(Z), (int)fl);
+                }
+                sxy[k] = make_int2(X, Y);
+                clip[k] = SLOW ? v : make_float4(v.x, v.y, v.w, Z);
+            }
             if (tri_words) {
 #pragma unroll
                 for (int q = 0; q < 3; ++q)
@@ -893,19 +998,19 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
                 // queued together when the warp has reconverged.
                 JobList jobs;
                 jobs.count = 0;
-                for (uint32_t tb = 0; tb < tc; tb += 32) {
+                for (uint32_t tb = H.t0; tb < tc; tb += 32) {
                     const uint32_t t = tb + (uint32_t)lane;
                     if (t < tc) {
                         TriClass k;
                         const uint32_t i0 = sidx8[3 * t], i1 = sidx8[3 * t + 1], i2 = sidx8[3 * t + 2];
-                        const int kind = classify<true>(i0, i1, i2, vc, svtx, clip, double_sided, tdet, c, d, k);
+                        const int kind = classify<true>(i0, i1, i2, vc, sxy, szf, clip, double_sided, tdet, c, d, k);
                         if (kind == kSlowClip) {
                             raster_clipped(clip[i0], clip[i1], clip[i2],
-                                           (((uint32_t)k.q0.w | (uint32_t)k.q1.w | (uint32_t)k.q2.w) & (OC_ZLO | OC_ZHI)) != 0,
+                                           ((uint32_t)(k.f0.y | k.f1.y | k.f2.y) & (OC_ZLO | OC_ZHI)) != 0,
                                            (d << 7) | t, c, jobs);
                         } else if (kind == kSlowSetup) {
-                            setup_and_raster(k.q0.x, k.q0.y, __int_as_float(k.q0.z), k.q1.x, k.q1.y,
-                                             __int_as_float(k.q1.z), k.q2.x, k.q2.y, __int_as_float(k.q2.z),
+                            setup_and_raster(k.q0.x, k.q0.y, __int_as_float(k.f0.x), k.q1.x, k.q1.y,
+                                             __int_as_float(k.f1.x), k.q2.x, k.q2.y, __int_as_float(k.f2.x),
                                              (d << 7) | t, c, jobs);
                         }
                     }
@@ -913,37 +1018,43 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
                     flush_jobs(jobs, c, lane);
                 }
             } else {
-                // Pre-filter 32 triangles per round (outcodes, snap, a pixel
-                // centre in the bbox); the candidates are compacted into a
-                // ring so that the backface, area and size tests, the setup and
-                // the raster run on full warps (at most about a quarter of the
-                // triangles of a dense meshlet have a sample in their bbox).
+                // Pre-filter 32 triangles per round (a pixel centre in the
+                // bbox; outcodes and snap flags where a vertex is outside the
+                // view volume); the candidates are compacted so that the
+                // backface, area and size tests, the setup and the raster run
+                // on full warps (at most about a quarter of the triangles of
+                // a dense meshlet have a sample in their bbox).
                 uint8_t* ring = s_ring[warp];
-                uint32_t head = 0, pending = 0;
-                for (uint32_t tbase = 0; tbase < tc; tbase += 32) {
+                uint32_t pending = 0;
+                for (uint32_t tbase = H.t0; tbase < tc; tbase += 32) {
                     const uint32_t t = tbase + lane;
-                    int kind = 0;
-                    if (t < tc) kind = prefilter(sidx8[3 * t], sidx8[3 * t + 1], sidx8[3 * t + 2], vc, svtx, c, d);
-                    any_slow |= kind == 2;
-                    const uint32_t fm = __ballot_sync(0xffffffffu, kind == 1);
-                    if (kind == 1) ring[(head + pending + __popc(fm & ((1u << lane) - 1u))) & 63u] = (uint8_t)t;
-                    pending += __popc(fm);
-                    const bool last = tbase + 32 >= tc;
-                    while (pending >= 32 || (last && pending > 0)) {
-                        __syncwarp();
-                        const uint32_t n = min(pending, 32u);
-                        const uint32_t ct = lane < n ? ring[(head + lane) & 63u] : 0xffffffffu;
-                        __syncwarp();
-                        any_slow |= raster_small(ct, sidx8, svtx, clip, double_sided, tdet, d, c, recs, ends, lane);
-                        head = (head + n) & 63u;
-                        pending -= n;
+                    bool cand = false;
+                    if (t < tc) {
+                        const uint32_t i0 = sidx8[3 * t], i1 = sidx8[3 * t + 1], i2 = sidx8[3 * t + 2];
+                        if (max(i0, max(i1, i2)) >= vc) {
+                            report(P.status, kStatusBadIndex, d);
+                        } else if (plain) {
+                            cand = covers_centre(sxy[i0], sxy[i1], sxy[i2]);
+                        } else {
+                            const int kind = prefilter(i0, i1, i2, sxy, szf, c);
+                            cand = kind == 1;
+                            any_slow |= kind == 2;
+                        }
                     }
+                    const uint32_t fm = __ballot_sync(0xffffffffu, cand);
+                    if (cand) ring[pending + __popc(fm & ((1u << lane) - 1u))] = (uint8_t)t;
+                    pending += __popc(fm);
+                }
+                __syncwarp();
+                for (uint32_t at = 0; at < pending; at += 32) {
+                    const uint32_t ct = at + lane < pending ? ring[at + lane] : 0xffffffffu;
+                    any_slow |= raster_small(ct, sidx8, sxy, clip, double_sided, tdet, d, c, recs, starts, lane);
                 }
             }
             if (!SLOW && __any_sync(0xffffffffu, any_slow) && lane == 0) {
                 const uint32_t k = atomicAdd(&V.counters[slot], 1u);
                 if (k < defer_cap)
-                    V.deferred[k] = d;
+                    V.deferred[k] = !(H.flags & kSplit) ? d : (d | ((uint32_t)H.t0 / 32u << kDeferPartShift) | kDeferSplit);
                 else
                     report(P.status, kStatusListOverflow, d);
             }
@@ -1007,17 +1118,27 @@ __global__ void __launch_bounds__(256) k_raster_big(const BigTri* __restrict__ q
     }
 }
 
+// Meshlets that a launch splits (see k_raster).
+uint32_t raster_split(uint32_t sm_count) { return sm_count * VKGV_RASTER_SPLIT_PER_SM; }
+
 // One wave of CTAs: every warp stays resident and takes work until none is
 // left.
 template <int WARPS>
-void launch_variant(const RasterParams& P, uint32_t sm_count, uint32_t blocks_override, cudaStream_t stream) {
+void launch_variant(RasterParams P, uint32_t sm_count, uint32_t blocks_override, cudaStream_t stream) {
     const uint32_t fast = blocks_override ? blocks_override : sm_count * (VKGV_RASTER_WARPS_PER_SM / WARPS);
     const uint32_t slow = blocks_override ? blocks_override : sm_count * (16 / WARPS > 0 ? 16 / WARPS : 1);
+    P.split = raster_split(sm_count);
     launch_pdl(k_raster<WARPS, false>, dim3(fast), dim3(WARPS * 32), 0, stream, P);
     launch_pdl(k_raster<WARPS, true>, dim3(slow), dim3(WARPS * 32), 0, stream, P);
 }
 
 }  // namespace
+
+uint32_t deferred_capacity(uint32_t draw_count, uint32_t sm_count) {
+    // every meshlet once, and the split ones once a round
+    const uint32_t split = raster_split(sm_count);
+    return draw_count + (kParts - 1) * (draw_count < split ? draw_count : split);
+}
 
 void launch_raster(const SceneArgs& S, const DeviceView* views, uint32_t nviews, const RasterLists& lists,
                    const RasterConfig& cfg, BigTri* big, uint32_t* big_count, uint32_t big_capacity,
@@ -1030,6 +1151,7 @@ void launch_raster(const SceneArgs& S, const DeviceView* views, uint32_t nviews,
     P.big_cap = big_capacity;
     P.small_area = cfg.small_area;
     P.chunk = cfg.chunk;
+    P.deferred_cap = deferred_capacity(S.draw_count, sm_count);
     P.status = status;
     P.work = work;
     for (uint32_t v0 = 0; v0 < nviews; v0 += kRasterMaxViews) {
