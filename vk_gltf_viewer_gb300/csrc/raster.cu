@@ -315,6 +315,10 @@ __device__ __noinline__ void raster_clipped(float4 v0, float4 v1, float4 v2, boo
         setup_and_raster(X[0], Y[0], Z[0], X[k], Y[k], Z[k], X[k + 1], Y[k + 1], Z[k + 1], id, c, jobs);
 }
 
+// Items a warp takes at once, at most (256-view torus grid 32.1 ms; 16: 32.4;
+// 8: 33.1).
+constexpr uint32_t kMaxRun = 32;
+
 // Views per raster launch (the launcher splits larger batches).
 constexpr uint32_t kRasterMaxViews = 1024;
 
@@ -710,12 +714,9 @@ template <int WARPS, bool SLOW>
 __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER_SM) / WARPS) k_raster(RasterParams P) {
     pdl_begin();
     // per vertex: clip {x, y, z, w} (slow instance) or clip {x, y, w} and the
-    // snapped depth (fast instance); the snapped {X, Y} (28.8); {depth bits,
-    // flags}, which the fast instance reads only for a meshlet that is not
-    // entirely inside the view volume
+    // snapped depth (fast instance); the snapped {X, Y} (28.8)
     __shared__ float4 s_clip[WARPS][64];
     __shared__ int2 s_xy[WARPS][64];
-    __shared__ int2 s_zf[WARPS][64];
     // the meshlet's triangle-index bytes (<= 126 triangles)
     __shared__ uint32_t s_idx[WARPS][96];
     __shared__ TriRec s_tri[WARPS][32];
@@ -727,7 +728,10 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
     __shared__ float s_vp[WARPS][16];
     // exclusive prefix of the views' work counts: view v owns the global
     // work items [s_pre[v], s_pre[v + 1])
-    __shared__ uint32_t s_pre[kRasterMaxViews + 1];
+    // (sized by the launch: with the flags sharing the records' memory, 20 KB a
+    // CTA instead of 25, which leaves more L1: the 1080p torus grid's frame
+    // 308.0 -> 305.6 us)
+    extern __shared__ uint32_t s_pre[];  // nviews + 1
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t nv = P.nviews;
     for (uint32_t v = threadIdx.x; v < nv; v += blockDim.x) {
@@ -766,7 +770,11 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
     const uint32_t defer_cap = P.deferred_cap;
     float4* clip = s_clip[warp];
     int2* sxy = s_xy[warp];
-    int2* szf = s_zf[warp];
+    // {depth bits, flags} of every vertex, which the fast instance reads only
+    // for a meshlet that is not entirely inside the view volume, before it
+    // writes a record
+    static_assert(sizeof(s_tri[0]) >= 64 * sizeof(int2), "vertex flags share the records' memory");
+    int2* szf = reinterpret_cast<int2*>(s_tri[warp]);
     uint32_t* sidx = s_idx[warp];
     const uint8_t* sidx8 = reinterpret_cast<const uint8_t*>(sidx);
     TriRec* recs = s_tri[warp];
@@ -775,7 +783,7 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
     // views are drawn roughly in order (their depth buffers stay in L2) and
     // no warp idles while work is left.
     const uint32_t warps_total = gridDim.x * WARPS;
-    const uint32_t grab = max(1u, min(32u, total / (warps_total * 8u)));
+    const uint32_t grab = max(1u, min(kMaxRun, total / (warps_total * 8u)));
     uint32_t cur_v = 0xffffffffu, cur_t = 0xffffffffu;  // view and node of s_vp / s_mvp
     const DeviceView* Vp = P.views;
     // the warp's raster context lives in shared memory (fewer live registers)
@@ -791,9 +799,9 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
     }
     // Per-meshlet headers of the current run, resolved one item per lane so
     // that the dependent loads (list entry -> draw -> primitive -> meshlet
-    // record, material) of up to 32 meshlets are in flight together instead
+    // record, material) of up to kMaxRun meshlets are in flight together instead
     // of one meshlet after another.
-    __shared__ ItemHeader s_hdr[WARPS][32];
+    __shared__ ItemHeader s_hdr[WARPS][kMaxRun];
     ItemHeader* hdr = s_hdr[warp];
     // the next run is requested while the current one is drawn, so the
     // atomic's round trip is off the critical path
@@ -868,7 +876,7 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
                 if (bad) report(P.status, kStatusBadIndex, d);
             }
             __syncwarp();  // every lane is done with the previous run's headers
-            hdr[lane] = h;
+            if (lane < (int)kMaxRun) hdr[lane] = h;
         }
         __syncwarp();
         for (uint32_t k = 0; k < stop - base; ++k) {
@@ -1128,8 +1136,9 @@ void launch_variant(RasterParams P, uint32_t sm_count, uint32_t blocks_override,
     const uint32_t fast = blocks_override ? blocks_override : sm_count * (VKGV_RASTER_WARPS_PER_SM / WARPS);
     const uint32_t slow = blocks_override ? blocks_override : sm_count * (16 / WARPS > 0 ? 16 / WARPS : 1);
     P.split = raster_split(sm_count);
-    launch_pdl(k_raster<WARPS, false>, dim3(fast), dim3(WARPS * 32), 0, stream, P);
-    launch_pdl(k_raster<WARPS, true>, dim3(slow), dim3(WARPS * 32), 0, stream, P);
+    const size_t pre = sizeof(uint32_t) * (P.nviews + 1);
+    launch_pdl(k_raster<WARPS, false>, dim3(fast), dim3(WARPS * 32), pre, stream, P);
+    launch_pdl(k_raster<WARPS, true>, dim3(slow), dim3(WARPS * 32), pre, stream, P);
 }
 
 }  // namespace
