@@ -52,9 +52,13 @@ struct RasterCtx {
     uint32_t* status;
 };
 
-// The depth test: a 64-bit max whose result is not needed (a reduction
-// that does not wait for the L2 round trip).
-__device__ __forceinline__ void plot(unsigned long long* p, unsigned long long v) { atomicMax(p, v); }
+// The depth test: a 64-bit max whose result is not needed.  atomicMax on the
+// view's pointer (which could point anywhere) compiles to an atomic with a
+// reply; the reduction on global memory sends none (1080p torus grid's frame
+// 306.8 -> 296.7 us, 4K 696 -> 673 us).
+__device__ __forceinline__ void plot(unsigned long long* p, unsigned long long v) {
+    asm volatile("red.relaxed.gpu.global.max.u64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "l"(v) : "memory");
+}
 
 __device__ void raster_rect(const int32_t* X, const int32_t* Y, const int32_t* bias, float z0, float pa, float pb,
                             uint32_t id, int px0, int py0, int px1, int py1, unsigned long long* depth,
