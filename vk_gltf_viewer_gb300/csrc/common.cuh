@@ -90,8 +90,10 @@ struct BigTri {
     uint32_t id;              // visbuffer id
     uint16_t px0, py0, px1, py1;  // inclusive pixel rectangle
     uint32_t view;
-    uint32_t _pad;
+    uint32_t flags;           // bits 0-2: edge biases (1: not top-left); kBigNarrow
 };
+// Every edge vector of the triangle is below 2^15 (128 pixels) on both axes.
+constexpr uint32_t kBigNarrow = 8;
 static_assert(sizeof(BigTri) == 56, "BigTri layout");
 
 // ------------------------------------------------------------ pinned math

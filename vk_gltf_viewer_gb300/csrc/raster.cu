@@ -121,6 +121,15 @@ struct JobList {
 __device__ void queue_job(const BinJob& j, uint32_t at, const RasterCtx& c) {
     const int64_t cs = c.chunk;
     const int64_t ncx = ((int64_t)(j.px1 - j.px0 + 1) + cs - 1) / cs;
+    uint32_t flags = kBigNarrow;
+    int32_t bias[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int32_t dx = j.x[(k + 1) % 3] - j.x[k], dy = j.y[(k + 1) % 3] - j.y[k];
+        bias[k] = (dy < 0 || (dy == 0 && dx > 0)) ? 0 : 1;
+        flags |= (uint32_t)bias[k] << k;
+        if (max(abs(dx), abs(dy)) >= 1 << 15) flags &= ~kBigNarrow;
+    }
     for (uint32_t i = 0; i < j.n; ++i, ++at) {
         const int64_t cx = i % ncx, cy = i / ncx;
         const int qx0 = (int)(j.px0 + cx * cs), qy0 = (int)(j.py0 + cy * cs);
@@ -134,16 +143,10 @@ __device__ void queue_job(const BinJob& j, uint32_t at, const RasterCtx& c) {
             t.id = j.id;
             t.px0 = (uint16_t)qx0, t.py0 = (uint16_t)qy0, t.px1 = (uint16_t)qx1, t.py1 = (uint16_t)qy1;
             t.view = c.view;
-            t._pad = 0;
+            t.flags = flags;
             c.big[at] = t;
         } else {
             report(c.status, kStatusQueueOverflow, at);
-            int32_t bias[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const int32_t dx = j.x[(k + 1) % 3] - j.x[k], dy = j.y[(k + 1) % 3] - j.y[k];
-                bias[k] = (dy < 0 || (dy == 0 && dx > 0)) ? 0 : 1;
-            }
             raster_rect(j.x, j.y, bias, j.z0, j.pa, j.pb, j.id, qx0, qy0, qx1, qy1, c.depth, c.w);
         }
     }
@@ -656,7 +659,7 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
                 t.px0 = (uint16_t)px0, t.py0 = (uint16_t)py0;
                 t.px1 = (uint16_t)(px0 + bw - 1u), t.py1 = (uint16_t)(py0 + coop_area / bw - 1u);
                 t.view = c.view;
-                t._pad = 0;
+                t.flags = ((rec.bits >> 7) & 7u) | kBigNarrow;
                 c.big[slot] = t;
                 coop_area = 0;
             } else {
@@ -1084,48 +1087,107 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
     }
 }
 
-// Drains the binned rectangles: one warp per rectangle, its pixels spread
-// over the lanes in row-major order (eight rectangles in flight per CTA).
-__global__ void __launch_bounds__(256) k_raster_big(const BigTri* __restrict__ q, const uint32_t* count,
-                                                    uint32_t cap, const DeviceView* __restrict__ views) {
+// A rectangle of a narrow triangle, set up by one lane and drawn by its warp.
+struct __align__(16) BigRect {
+    int32_t e[3];       // edge values at the rectangle's first pixel centre, clamped, biases subtracted
+    uint32_t d[3];      // edge vectors: x | y << 16
+    float z0, pa, pb;   // depth plane
+    uint32_t id;
+    int32_t x, y;       // first pixel centre - vertex 0
+    uint32_t width;     // 2^18 / width rounded up (19) | width (7)
+    uint32_t area;      // (13) | the view's row pitch in pixels << 16
+    unsigned long long* at;
+};
+
+// Drains the binned rectangles, each warp up to 32 of them at a time: a lane
+// sets up one rectangle (edge values at its corner), then the warp draws them
+// one after another, its lanes over a rectangle's pixels in row-major order.
+// Issue-bound: set up by all lanes alike, a rectangle of some 34 pixels took
+// 160 instructions, most of them setup (119,000 rectangles of the 1080p torus
+// grid 34.1 -> 23.5 us).  Runs of neighbouring rectangles instead of every
+// warps-th: 31 us.
+constexpr int kBigWarps = 8;
+__global__ void __launch_bounds__(32 * kBigWarps) k_raster_big(const BigTri* __restrict__ q, const uint32_t* count,
+                                                               uint32_t cap, const DeviceView* __restrict__ views) {
     pdl_begin();
+    __shared__ BigRect s_rect[kBigWarps][32];
     const uint32_t n = min(*count, cap);
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t e = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); e < n; e += warps) {
-        const BigTri t = q[e];
-        const DeviceView& V = views[t.view];
-        unsigned long long* depth = V.depth_id;
-        const uint32_t w = V.w;
-        const unsigned long long lo = (unsigned long long)t.id + 1ull;
-        int32_t bias[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const int a = k, b = (k + 1) % 3;
-            const int32_t dx = t.x[b] - t.x[a], dy = t.y[b] - t.y[a];
-            bias[k] = (dy < 0 || (dy == 0 && dx > 0)) ? 0 : 1;
-        }
-        const uint32_t bw = (uint32_t)t.px1 - t.px0 + 1u, area = bw * ((uint32_t)t.py1 - t.py0 + 1u);
-        // floor((i + 0.5) / bw) from the float reciprocal is exact here: the
-        // quotient stays at least 0.5 / bw from an integer and i < 4096.
-        const float inv_bw = 1.0f / (float)bw;
-        for (uint32_t i = lane; i < area; i += 32) {
-            const uint32_t ly = (uint32_t)(((float)i + 0.5f) * inv_bw);
-            const int px = (int)(t.px0 + (i - ly * bw)), py = (int)(t.py0 + ly);
-            const int32_t sx = px * 256 + 128, sy = py * 256 + 128;
-            bool covered = true;
+    BigRect* rects = s_rect[threadIdx.x >> 5];
+    const uint32_t warps = gridDim.x * kBigWarps;
+    // Each warp takes every warps-th rectangle (the pieces of one large triangle
+    // are neighbours in the queue), 32 of them at a time.
+    for (uint32_t first = blockIdx.x * kBigWarps + (threadIdx.x >> 5); first < n; first += 32 * warps) {
+        const uint32_t here = min(32u, (n - first + warps - 1) / warps);
+        bool wide = false;
+        __syncwarp();  // the previous ones are drawn
+        if (lane < here) {
+            const BigTri t = q[first + lane * warps];
+            const DeviceView& V = views[t.view];
+            const uint32_t bw = (uint32_t)t.px1 - t.px0 + 1u;
+            wide = !(t.flags & kBigNarrow);
+            const int32_t cx = ((int32_t)t.px0 << 8) + 128, cy = ((int32_t)t.py0 << 8) + 128;
+            BigRect r;
+            // Over at most 64 x 64 pixels a narrow triangle's edge value moves
+            // by less than 2^30, so the corner's value may be clamped to that
+            // without a change of any sign.
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                const int a = k, b = (k + 1) % 3;
-                const int64_t ev = (int64_t)(t.x[b] - t.x[a]) * (sy - t.y[a]) -
-                                   (int64_t)(t.y[b] - t.y[a]) * (sx - t.x[a]);
-                covered = covered && ev >= bias[k];
+                const int32_t dx = t.x[(k + 1) % 3] - t.x[k], dy = t.y[(k + 1) % 3] - t.y[k];
+                const int64_t c = (int64_t)dx * (cy - t.y[k]) - (int64_t)dy * (cx - t.x[k]) - (int32_t)((t.flags >> k) & 1u);
+                constexpr int64_t kLim = 1 << 30;
+                r.e[k] = (int32_t)(c < -kLim ? -kLim : (c > kLim ? kLim : c));
+                r.d[k] = ((uint32_t)dx & 0xFFFFu) | ((uint32_t)dy << 16);
             }
-            if (!covered) continue;
-            float z = __fmaf_rn(t.pa, __int2float_rn(sx - t.x[0]), __fmaf_rn(t.pb, __int2float_rn(sy - t.y[0]), t.z0));
-            if (!(z > 0.0f)) z = 0.0f;
-            if (z > 1.0f) z = 1.0f;
-            plot(depth + (size_t)py * w + px, ((unsigned long long)__float_as_uint(z) << 32) | lo);
+            r.z0 = t.z0, r.pa = t.pa, r.pb = t.pb;
+            r.id = t.id;
+            r.x = cx - t.x[0], r.y = cy - t.y[0];
+            // floor(i / bw) by a reciprocal rounded up, exact for i < 4096 and
+            // bw <= 64: i times its error, below 4096 / 2^18, stays under 1 / bw
+            // (whole only for the powers of two, where it is exact)
+            r.width = __float2uint_ru(fmul(262144.0f, __frcp_rn((float)bw))) | (bw << 19);
+            r.area = (wide ? 0u : bw * ((uint32_t)t.py1 - t.py0 + 1u)) | (V.w << 16);
+            r.at = V.depth_id + (size_t)t.py0 * V.w + t.px0;
+            rects[lane] = r;
+        }
+        unsigned wides = __ballot_sync(0xffffffffu, wide);
+        for (uint32_t j = 0; j < here; ++j) {
+            const BigRect r = rects[j];
+            const uint32_t area = r.area & 0xFFFFu, w = r.area >> 16;
+            const int32_t dx0 = (int32_t)(int16_t)(r.d[0] & 0xFFFFu), dy0 = (int32_t)r.d[0] >> 16;
+            const int32_t dx1 = (int32_t)(int16_t)(r.d[1] & 0xFFFFu), dy1 = (int32_t)r.d[1] >> 16;
+            const int32_t dx2 = (int32_t)(int16_t)(r.d[2] & 0xFFFFu), dy2 = (int32_t)r.d[2] >> 16;
+            const uint32_t inv = r.width & 0x7FFFFu, bw = r.width >> 19;
+            for (uint32_t i = lane; i < area; i += 32) {
+                const uint32_t ly = (i * inv) >> 18, lx = i - ly * bw;
+                const int32_t sx = (int32_t)(lx << 8), sy = (int32_t)(ly << 8);
+                const int32_t a = r.e[0] + sy * dx0 - sx * dy0, b = r.e[1] + sy * dx1 - sx * dy1;
+                const int32_t c = r.e[2] + sy * dx2 - sx * dy2;
+                if ((a | b | c) >= 0)
+                    plot(r.at + (size_t)ly * w + lx,
+                         fragment(r.pa, r.pb, r.z0, __int2float_rn(r.x + sx), __int2float_rn(r.y + sy), r.id));
+            }
+        }
+        // triangles of 128 pixels and more: every edge value in 64 bits
+        for (; wides; wides &= wides - 1) {
+            const BigTri t = q[first + ((uint32_t)__ffs((int)wides) - 1u) * warps];
+            const DeviceView& V = views[t.view];
+            const uint32_t bw = (uint32_t)t.px1 - t.px0 + 1u, area = bw * ((uint32_t)t.py1 - t.py0 + 1u);
+            const uint32_t inv = __float2uint_ru(fmul(262144.0f, __frcp_rn((float)bw)));
+            for (uint32_t i = lane; i < area; i += 32) {
+                const uint32_t ly = (i * inv) >> 18, px = t.px0 + (i - ly * bw), py = t.py0 + ly;
+                const int32_t sx = (int32_t)(px << 8) + 128, sy = (int32_t)(py << 8) + 128;
+                bool covered = true;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const int64_t ev = (int64_t)(t.x[(k + 1) % 3] - t.x[k]) * (sy - t.y[k]) -
+                                       (int64_t)(t.y[(k + 1) % 3] - t.y[k]) * (sx - t.x[k]);
+                    covered = covered && ev >= (int64_t)((t.flags >> k) & 1u);
+                }
+                if (covered)
+                    plot(V.depth_id + (size_t)py * V.w + px,
+                         fragment(t.pa, t.pb, t.z0, __int2float_rn(sx - t.x[0]), __int2float_rn(sy - t.y[0]), t.id));
+            }
         }
     }
 }
@@ -1189,11 +1251,11 @@ void launch_raster(const SceneArgs& S, const DeviceView* views, uint32_t nviews,
     cudaGetDevice(&dev);
     int per_sm = dev >= 0 && dev < 64 ? resident[dev].load(std::memory_order_relaxed) : 0;
     if (per_sm <= 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_raster_big, 256, 0) != cudaSuccess || per_sm <= 0)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_raster_big, 32 * kBigWarps, 0) != cudaSuccess || per_sm <= 0)
             per_sm = 4;
         if (dev >= 0 && dev < 64) resident[dev].store(per_sm, std::memory_order_relaxed);
     }
-    launch_pdl(k_raster_big, dim3(sm_count * (uint32_t)per_sm), dim3(256), 0, stream, (const BigTri*)big,
+    launch_pdl(k_raster_big, dim3(sm_count * (uint32_t)per_sm), dim3(32 * kBigWarps), 0, stream, (const BigTri*)big,
                (const uint32_t*)big_count, big_capacity, views);
 }
 
