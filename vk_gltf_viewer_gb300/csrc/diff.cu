@@ -235,6 +235,15 @@ __device__ __forceinline__ void clip_ab(const float* VP, const float* q, float n
     b = __fadd_rn(__fmaf_rn(-ny, wh, yh), __fmaf_rn(-ny, wl, yl));
 }
 
+// Adds into a float4 accumulator without waiting for the sum.  atomicAdd on
+// the argument's generic pointer compiles to an atomic with a reply (64 views
+// of 512^2, a step: 716 -> 634 us; 128 views of 1.3M triangles: 3.62 -> 3.35 ms).
+__device__ __forceinline__ void accumulate(float4* p, float x, float y, float z) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(p)), "f"(x),
+                 "f"(y), "f"(z), "f"(0.0f)
+                 : "memory");
+}
+
 // One pixel of the forward image (BACKWARD = false) or of the gradient pass,
 // which in a captured forward + backward step (A.write_rgb) writes the image
 // too: the same operations in the same order, so the same bits.
@@ -346,10 +355,10 @@ __device__ __forceinline__ void shade_pixel(const DiffArgs& A, const DeviceView&
     if (A.acc_tex) {
         const float w00 = (1.0f - ax) * (1.0f - ay), w01 = ax * (1.0f - ay);
         const float w10 = (1.0f - ax) * ay, w11 = ax * ay;
-        atomicAdd(A.acc_tex + i00 / 3, make_float4(dtex[0] * w00, dtex[1] * w00, dtex[2] * w00, 0.0f));
-        atomicAdd(A.acc_tex + i01 / 3, make_float4(dtex[0] * w01, dtex[1] * w01, dtex[2] * w01, 0.0f));
-        atomicAdd(A.acc_tex + i10 / 3, make_float4(dtex[0] * w10, dtex[1] * w10, dtex[2] * w10, 0.0f));
-        atomicAdd(A.acc_tex + i11 / 3, make_float4(dtex[0] * w11, dtex[1] * w11, dtex[2] * w11, 0.0f));
+        accumulate(A.acc_tex + i00 / 3, dtex[0] * w00, dtex[1] * w00, dtex[2] * w00);
+        accumulate(A.acc_tex + i01 / 3, dtex[0] * w01, dtex[1] * w01, dtex[2] * w01);
+        accumulate(A.acc_tex + i10 / 3, dtex[0] * w10, dtex[1] * w10, dtex[2] * w10);
+        accumulate(A.acc_tex + i11 / 3, dtex[0] * w11, dtex[1] * w11, dtex[2] * w11);
     }
     // d tex / d uv' through the bilinear weights
     float dtu = 0.0f, dtv = 0.0f;
@@ -367,7 +376,7 @@ __device__ __forceinline__ void shade_pixel(const DiffArgs& A, const DeviceView&
     for (int k = 0; k < 3; ++k) {
         dlam[k] = dcol[0] * C[k][0] + dcol[1] * C[k][1] + dcol[2] * C[k][2] + du * UV[k][0] + dv * UV[k][1];
         if (A.acc_col)
-            atomicAdd(A.acc_col + vi[k], make_float4(dcol[0] * lam[k], dcol[1] * lam[k], dcol[2] * lam[k], 0.0f));
+            accumulate(A.acc_col + vi[k], dcol[0] * lam[k], dcol[1] * lam[k], dcol[2] * lam[k]);
     }
     if (!A.acc_pos) return;
     const float dot = lam[0] * dlam[0] + lam[1] * dlam[1] + lam[2] * dlam[2];
@@ -378,9 +387,8 @@ __device__ __forceinline__ void shade_pixel(const DiffArgs& A, const DeviceView&
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const float dx = da[k], dy = db[k], dw = -nx * da[k] - ny * db[k];
-        atomicAdd(A.acc_pos + vi[k], make_float4(VP[0] * dx + VP[1] * dy + VP[3] * dw,
-                                                 VP[4] * dx + VP[5] * dy + VP[7] * dw,
-                                                 VP[8] * dx + VP[9] * dy + VP[11] * dw, 0.0f));
+        accumulate(A.acc_pos + vi[k], VP[0] * dx + VP[1] * dy + VP[3] * dw, VP[4] * dx + VP[5] * dy + VP[7] * dw,
+                   VP[8] * dx + VP[9] * dy + VP[11] * dw);
     }
 }
 
