@@ -454,7 +454,8 @@ __global__ void __launch_bounds__(256, 3) k_diff_shade_chunks(DiffArgs A, const 
     const uint32_t total = s_pre[nviews];
     float sn, cs;
     sincosf(A.uv_rotation, &sn, &cs);
-    float VP[16];
+    __shared__ float s_vp[8][16];  // the view-projection of the warp's view
+    float* VP = s_vp[threadIdx.x >> 5];
     uint32_t cur = 0xffffffffu;
     float loss_acc = 0.0f;
     for (;;) {
@@ -474,14 +475,16 @@ __global__ void __launch_bounds__(256, 3) k_diff_shade_chunks(DiffArgs A, const 
         const DeviceView& V = views[v];
         if (v != cur) {
             cur = v;
-#pragma unroll
-            for (int k = 0; k < 16; ++k) VP[k] = V.cam->view_projection[k];
+            __syncwarp();
+            if ((threadIdx.x & 31u) < 16) VP[threadIdx.x & 31u] = V.cam->view_projection[threadIdx.x & 31u];
+            __syncwarp();
         }
         const uint32_t n = V.w * V.h, base = (item - s_pre[v]) * kShadeChunk;
-        // two pixels per step: the compiler interleaves their load chains
-        // (id -> vertex triple -> vertex records -> texels), and the kernel
-        // then fits 80 registers, three CTAs per SM (C5 step -1.2%)
-#pragma unroll 2
+        // one pixel per step: 80 registers without spills, three CTAs per SM,
+        // since the view-projection is in shared memory (64 views of 512^2, a
+        // step: 634 -> 584 us; two interleaved pixels 598; four CTAs, which
+        // spill, 604; 128 views of 1.3M triangles 3.35 -> 3.21 ms)
+#pragma unroll 1
         for (uint32_t j = threadIdx.x & 31u; j < kShadeChunk; j += 32) {
             const uint32_t p = base + j;
             if (p < n) shade_pixel<BACKWARD>(A, V, VP, sn, cs, p, loss_acc);
