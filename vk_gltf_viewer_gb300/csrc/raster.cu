@@ -48,7 +48,7 @@ struct RasterCtx {
     uint32_t* big_count;
     uint32_t big_cap;
     uint32_t small_area;
-    uint32_t chunk;
+    uint32_t chunk, chunk_log2;  // a power of two
     uint32_t* status;
 };
 
@@ -119,8 +119,8 @@ struct JobList {
 // The rectangles of one job, queued at c.big[at, at + n) (past the queue's
 // capacity they are drawn in place and the overflow is reported).
 __device__ void queue_job(const BinJob& j, uint32_t at, const RasterCtx& c) {
-    const int64_t cs = c.chunk;
-    const int64_t ncx = ((int64_t)(j.px1 - j.px0 + 1) + cs - 1) / cs;
+    const int32_t cs = (int32_t)c.chunk;
+    const uint32_t ncx = (uint32_t)(j.px1 - j.px0 + cs) >> c.chunk_log2;
     uint32_t flags = kBigNarrow;
     int32_t bias[3];
 #pragma unroll
@@ -130,11 +130,11 @@ __device__ void queue_job(const BinJob& j, uint32_t at, const RasterCtx& c) {
         flags |= (uint32_t)bias[k] << k;
         if (max(abs(dx), abs(dy)) >= 1 << 15) flags &= ~kBigNarrow;
     }
-    for (uint32_t i = 0; i < j.n; ++i, ++at) {
-        const int64_t cx = i % ncx, cy = i / ncx;
-        const int qx0 = (int)(j.px0 + cx * cs), qy0 = (int)(j.py0 + cy * cs);
-        const int qx1 = (int)min((int64_t)j.px1, j.px0 + (cx + 1) * cs - 1);
-        const int qy1 = (int)min((int64_t)j.py1, j.py0 + (cy + 1) * cs - 1);
+    uint32_t cx = 0;
+    int32_t qx0 = j.px0, qy0 = j.py0;
+    for (uint32_t i = 0; i < j.n; ++i, ++at, ++cx, qx0 += cs) {
+        if (cx == ncx) cx = 0, qx0 = j.px0, qy0 += cs;
+        const int32_t qx1 = min(j.px1, qx0 + cs - 1), qy1 = min(j.py1, qy0 + cs - 1);
         if (at < c.big_cap) {
             BigTri t;
             t.x[0] = j.x[0], t.x[1] = j.x[1], t.x[2] = j.x[2];
@@ -222,15 +222,14 @@ __device__ __noinline__ void setup_and_raster(int32_t X0, int32_t Y0, float Z0, 
         raster_rect(X, Y, bias, Z0, pa, pb, id, (int)px0, (int)py0, (int)px1, (int)py1, c.depth, c.w);
         return;
     }
-    const int64_t cs = c.chunk;
-    const int64_t ncx = (bw + cs - 1) / cs, ncy = (bh + cs - 1) / cs;
+    const uint32_t ncx = (uint32_t)(bw + c.chunk - 1) >> c.chunk_log2, ncy = (uint32_t)(bh + c.chunk - 1) >> c.chunk_log2;
     BinJob j;
     j.x[0] = X0, j.x[1] = X1, j.x[2] = X2;
     j.y[0] = Y0, j.y[1] = Y1, j.y[2] = Y2;
     j.z0 = Z0, j.pa = pa, j.pb = pb;
     j.id = id;
     j.px0 = (int32_t)px0, j.py0 = (int32_t)py0, j.px1 = (int32_t)px1, j.py1 = (int32_t)py1;
-    j.n = (uint32_t)(ncx * ncy);
+    j.n = ncx * ncy;
     if (jobs.count < kMaxJobs) {
         jobs.job[jobs.count++] = j;
     } else {
@@ -773,6 +772,7 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
     // (and the longest of them takes one round, not four), and at the end of
     // a long one the last warps are not left alone with whole heavy meshlets.
     const uint32_t total = s_pre[nv] + (kParts - 1) * min(s_pre[nv], P.split);
+    if (total == 0) return;  // no CTA takes anything: the work counters stay at zero
     const uint32_t slot = P.lists.deferred_slot;
     const uint32_t defer_cap = P.deferred_cap;
     float4* clip = s_clip[warp];
@@ -802,6 +802,7 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
         c.big_cap = P.big_cap;
         c.small_area = P.small_area;
         c.chunk = P.chunk;
+        c.chunk_log2 = 31u - (uint32_t)__clz((int)P.chunk);
         c.status = P.status;
     }
     // Per-meshlet headers of the current run, resolved one item per lane so
