@@ -19,6 +19,9 @@ namespace {
 // (-1,-1,-1), (1,-1,1), (1,1,1), (-1,-1,1), (-1,1,1).
 constexpr uint32_t kCornerSigns = 0x2c2f66;
 
+// Mips of the largest pyramid (13: of an 8192 x 8192 view).
+constexpr uint32_t kMaxMips = 16;
+
 // Exact floor(log2(m)) clamped to [0, levels-1]; m <= 0 or NaN -> 0,
 // +inf -> levels-1.
 __device__ __forceinline__ int hiz_level(float m, uint32_t levels) {
@@ -38,7 +41,7 @@ __device__ __forceinline__ int hiz_level(float m, uint32_t levels) {
 // same integer footprint and fp32 products.
 // An occluding footprint is reported in *foot: level << 28 | a0 << 16 |
 // b0 << 4 | (a1 - a0) << 2 | (b1 - b0).
-__device__ __forceinline__ bool fine_occluded(const float* pyr, uint32_t pw0, uint32_t ph0, uint32_t plevels,
+__device__ __forceinline__ bool fine_occluded(const float* pyr, const uint32_t* mips, uint32_t pw0, uint32_t ph0, uint32_t plevels,
                                               uint32_t vw, uint32_t vh, float mn0, float mx0, float mn1, float mx1,
                                               float mx2, uint32_t* foot) {
     if ((vw & 1u) || (vh & 1u) || vw == 0 || vh == 0) return false;
@@ -55,7 +58,7 @@ __device__ __forceinline__ bool fine_occluded(const float* pyr, uint32_t pw0, ui
         const int a0 = i0 >> l, a1 = i1 >> l, b0 = j0 >> l, b1 = j1 >> l;
         if (a1 - a0 > 3 || b1 - b0 > 3) continue;
         const uint32_t mw = mip_dim(pw0, (uint32_t)l);
-        const float* img = pyr + mip_offset(pw0, ph0, (uint32_t)l);
+        const float* img = pyr + mips[l];
         for (int y = b0; y <= b1; ++y)
             for (int x = a0; x <= a1; ++x)
                 if (__ldg(img + (size_t)y * mw + x) < mx2) return false;
@@ -68,16 +71,27 @@ __device__ __forceinline__ bool fine_occluded(const float* pyr, uint32_t pw0, ui
 
 // Repeats a fine footprint (the low word of a fine key) on a pyramid of the
 // same shape: occluded iff every texel is >= mx2.
-__device__ __forceinline__ bool footprint_occluded(uint32_t foot, float mx2, const float* pyr, uint32_t pw0,
-                                                   uint32_t ph0) {
+__device__ __forceinline__ bool footprint_occluded(uint32_t foot, float mx2, const float* pyr, const uint32_t* mips,
+                                                   uint32_t pw0) {
     const uint32_t l = foot >> 28, a0 = (foot >> 16) & 0xfffu, b0 = (foot >> 4) & 0xfffu;
     const uint32_t a1 = a0 + ((foot >> 2) & 3u), b1 = b0 + (foot & 3u);
     const uint32_t mw = mip_dim(pw0, l);
-    const float* img = pyr + mip_offset(pw0, ph0, l);
+    const float* img = pyr + mips[l];
     for (uint32_t y = b0; y <= b1; ++y)
         for (uint32_t x = a0; x <= a1; ++x)
             if (__ldg(img + (size_t)y * mw + x) < mx2) return false;
     return true;
+}
+
+// A meshlet's cone: two 16-byte loads where the array allows them.
+__device__ __forceinline__ vkgv_meshlet_cone load_cone(uint64_t cones, uint32_t i) {
+    const vkgv_meshlet_cone* p = reinterpret_cast<const vkgv_meshlet_cone*>(cones) + i;
+    if (cones & 15u) return *p;
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    vkgv_meshlet_cone c;
+    c.center[0] = a.x, c.center[1] = a.y, c.center[2] = a.z, c.radius = a.w;
+    c.axis[0] = b.x, c.axis[1] = b.y, c.axis[2] = b.z, c.cutoff = b.w;
+    return c;
 }
 
 struct CullResult {
@@ -113,12 +127,12 @@ __device__ __forceinline__ unsigned long long pack_fine(float maxz, uint32_t foo
 
 // Repeats a packed lookup on a pyramid of the same shape: visible iff the
 // footprint's MIN depth is below the nearest AABB depth.
-__device__ __forceinline__ bool sample_visible(unsigned long long key, const float* pyr, uint32_t pw0, uint32_t ph0) {
+__device__ __forceinline__ bool sample_visible(unsigned long long key, const float* pyr, const uint32_t* mips, uint32_t pw0) {
     const uint32_t lo = (uint32_t)key;
     const float maxz = __uint_as_float((uint32_t)(key >> 32));
     const uint32_t lvl = lo >> 28, x0 = (lo >> 16) & 0xfffu, y0 = (lo >> 4) & 0xfffu;
     const uint32_t mw = mip_dim(pw0, lvl);
-    const float* img = pyr + mip_offset(pw0, ph0, lvl);
+    const float* img = pyr + mips[lvl];
     float depth = __ldg(img + (size_t)y0 * mw + x0);
     if (lo & 2u) depth = gmin(depth, __ldg(img + (size_t)y0 * mw + x0 + 1));
     if (lo & 1u) {
@@ -128,9 +142,9 @@ __device__ __forceinline__ bool sample_visible(unsigned long long key, const flo
     return depth < maxz;
 }
 
-__device__ __forceinline__ CullResult cull_one(const SceneArgs& S, const DeviceView& V, const float* frustum, const float* eye,
-                                               const float* occl_vp, const float* pyr, uint32_t pw0,
-                                               uint32_t ph0, uint32_t plevels, uint32_t flags, uint32_t d,
+__device__ __forceinline__ CullResult cull_one(const SceneArgs& S, const DeviceView& V, const float4* frustum, const float* eye,
+                                               const float4* occl_vp, const float* pyr, const uint32_t* mips,
+                                               uint32_t pw0, uint32_t ph0, uint32_t plevels, uint32_t flags, uint32_t d,
                                                bool retest, uint32_t* status) {
     CullResult res{false, false, 0ull};
     const vkgv_meshlet_draw dr = S.draws[d];
@@ -165,7 +179,8 @@ __device__ __forceinline__ CullResult cull_one(const SceneArgs& S, const DeviceV
     if ((flags & VKGV_CULL_FRUSTUM) && !retest) {
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
-            const float p0 = frustum[4 * i], p1 = frustum[4 * i + 1], p2 = frustum[4 * i + 2], p3 = frustum[4 * i + 3];
+            const float4 plane = frustum[i];
+            const float p0 = plane.x, p1 = plane.y, p2 = plane.z, p3 = plane.w;
             float radius = fadd(fadd(fmul(we[0], fabsf(p0)), fmul(we[1], fabsf(p1))), fmul(we[2], fabsf(p2)));
             float distance = fsub(fadd(fadd(fmul(p0, wc4[0]), fmul(p1, wc4[1])), fmul(p2, wc4[2])), p3);
             if (-radius > distance) return res;
@@ -178,7 +193,7 @@ __device__ __forceinline__ CullResult cull_one(const SceneArgs& S, const DeviceV
         !S.mats[prim->material_index].double_sided) {
         const uint64_t cones = S.cone_table[dr.primitive_index];
         if (cones) {
-            const vkgv_meshlet_cone& cone = reinterpret_cast<const vkgv_meshlet_cone*>(cones)[dr.meshlet_index];
+            const vkgv_meshlet_cone cone = load_cone(cones, dr.meshlet_index);
             bool culled;
             if (V.eyes && dr.transform_index < S.transform_count) {
                 const float4 o = __ldg(V.eyes + dr.transform_index);
@@ -202,12 +217,18 @@ __device__ __forceinline__ CullResult cull_one(const SceneArgs& S, const DeviceV
     const float ay[2] = {fadd(we[1], wc4[1]), fadd(-we[1], wc4[1])};
     const float az[2] = {fadd(we[2], wc4[2]), fadd(-we[2], wc4[2])};
     float rows[4][2][2][2];  // [j][x sign][y sign][z sign]
+    float vp[16];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 col = occl_vp[k];
+        vp[4 * k] = col.x, vp[4 * k + 1] = col.y, vp[4 * k + 2] = col.z, vp[4 * k + 3] = col.w;
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const float mx[2] = {fmul(occl_vp[0 * 4 + j], ax[0]), fmul(occl_vp[0 * 4 + j], ax[1])};
-        const float my[2] = {fmul(occl_vp[1 * 4 + j], ay[0]), fmul(occl_vp[1 * 4 + j], ay[1])};
-        const float mz[2] = {fmul(occl_vp[2 * 4 + j], az[0]), fmul(occl_vp[2 * 4 + j], az[1])};
-        const float m3 = fmul(occl_vp[3 * 4 + j], 1.0f);
+        const float mx[2] = {fmul(vp[0 * 4 + j], ax[0]), fmul(vp[0 * 4 + j], ax[1])};
+        const float my[2] = {fmul(vp[1 * 4 + j], ay[0]), fmul(vp[1 * 4 + j], ay[1])};
+        const float mz[2] = {fmul(vp[2 * 4 + j], az[0]), fmul(vp[2 * 4 + j], az[1])};
+        const float m3 = fmul(vp[3 * 4 + j], 1.0f);
 #pragma unroll
         for (int a = 0; a < 2; ++a)
 #pragma unroll
@@ -246,7 +267,7 @@ __device__ __forceinline__ CullResult cull_one(const SceneArgs& S, const DeviceV
     int lvl = hiz_level(gmax(width, height), plevels);
     float cx = fmul(fadd(mn0, mx0), 0.5f), cy = fmul(fadd(mn1, mx1), 0.5f);
     uint32_t mw = mip_dim(pw0, (uint32_t)lvl), mh = mip_dim(ph0, (uint32_t)lvl);
-    const float* img = pyr + mip_offset(pw0, ph0, (uint32_t)lvl);
+    const float* img = pyr + mips[lvl];
     int x0 = 0, x1 = 0, y0 = 0, y1 = 0;
     int nx = footprint_axis(cx, mw, x0, x1);
     int ny = footprint_axis(cy, mh, y0, y1);
@@ -261,7 +282,7 @@ __device__ __forceinline__ CullResult cull_one(const SceneArgs& S, const DeviceV
         res.occluded = true;
         res.sample = pack_sample(mx2, lvl, x0, x1, nx, y0, y1, ny);
     } else if ((flags & VKGV_CULL_OCCLUSION_FINE) && all_front &&
-               fine_occluded(pyr, pw0, ph0, plevels, V.w, V.h, mn0, mx0, mn1, mx1, mx2, &foot)) {
+               fine_occluded(pyr, mips, pw0, ph0, plevels, V.w, V.h, mn0, mx0, mn1, mx1, mx2, &foot)) {
         res.occluded = true;
         res.sample = pack_fine(mx2, foot);
     } else {
@@ -321,15 +342,24 @@ __global__ void __launch_bounds__(256, 5) k_cull(SceneArgs S, const DeviceView* 
     pdl_begin();
     const DeviceView& V = views[blockIdx.y];
     const vkgv_camera* cam = V.cam;
-    __shared__ float s_frustum[24];
-    __shared__ float s_vp[16];
+    // 16-byte words: one shared load a plane and a column instead of four, and
+    // no loop over the mips' sizes for a lookup (256 views of 843,776 draws: both
+    // passes 7.2 -> 6.95 ms, the frame 31.6 -> 31.3; 1080p 285.9 -> 283.5 us)
+    __shared__ float4 s_frustum[6];
+    __shared__ float4 s_vp[4];
+    __shared__ uint32_t s_mips[kMaxMips];  // the pyramid's mip offsets
     __shared__ float s_eye[3];
     __shared__ int s_eye_ok;
     __shared__ int s_same;
-    if (threadIdx.x < 24) s_frustum[threadIdx.x] = (&cam->frustum[0][0])[threadIdx.x];
+    if (threadIdx.x < 24) (&s_frustum[0].x)[threadIdx.x] = (&cam->frustum[0][0])[threadIdx.x];
     if (threadIdx.x < 16)
-        s_vp[threadIdx.x] = pass == 1 ? cam->prev_occlusion_view_projection[threadIdx.x]
-                                      : cam->occlusion_view_projection[threadIdx.x];
+        (&s_vp[0].x)[threadIdx.x] = pass == 1 ? cam->prev_occlusion_view_projection[threadIdx.x]
+                                              : cam->occlusion_view_projection[threadIdx.x];
+    if (threadIdx.x >= 96 && threadIdx.x < 96 + kMaxMips) {
+        const bool first = pass == 1;
+        s_mips[threadIdx.x - 96] = (uint32_t)mip_offset(first ? V.prev_w0 : V.w >> 1, first ? V.prev_h0 : V.h >> 1,
+                                                        threadIdx.x - 96);
+    }
     if (threadIdx.x == 32) {
         // the eye of the raster view-projection, for the cone test
         float vp[16];
@@ -394,9 +424,9 @@ __global__ void __launch_bounds__(256, 5) k_cull(SceneArgs S, const DeviceView* 
                     const unsigned long long key = V.reject_samples[i];
                     if (key >> 63) {
                         const float mz = __uint_as_float((uint32_t)(key >> 32) & 0x7fffffffu);
-                        if (footprint_occluded((uint32_t)key, mz, pyr, pw0, ph0)) verdict = 0;
+                        if (footprint_occluded((uint32_t)key, mz, pyr, s_mips, pw0)) verdict = 0;
                     } else {
-                        const bool coarse = sample_visible(key, pyr, pw0, ph0);
+                        const bool coarse = sample_visible(key, pyr, s_mips, pw0);
                         if (!coarse) verdict = 0;
                         else if (!(flags & VKGV_CULL_OCCLUSION_FINE)) verdict = 1;
                     }
@@ -404,7 +434,7 @@ __global__ void __launch_bounds__(256, 5) k_cull(SceneArgs S, const DeviceView* 
                 if (verdict >= 0) {
                     vis = verdict == 1;
                 } else {
-                    CullResult r = cull_one(S, V, s_frustum, eye, s_vp, pyr, pw0, ph0, pl, flags, d, pass == 2,
+                    CullResult r = cull_one(S, V, s_frustum, eye, s_vp, pyr, s_mips, pw0, ph0, pl, flags, d, pass == 2,
                                             status);
                     vis = r.visible;
                     occ = r.occluded;
