@@ -22,6 +22,18 @@ constexpr uint32_t kCornerSigns = 0x2c2f66;
 // Mips of the largest pyramid (13: of an 8192 x 8192 view).
 constexpr uint32_t kMaxMips = 16;
 
+// max(x, lo) then min(.., hi) that keep a NaN, as gclamp does (x is NaN where
+// a corner lies on the camera plane), in one instruction each: GLSL's
+// definitions compile to a compare and a select (with the bounds below and the
+// fine test's level found by its width, 256 views of 843,776 draws: both
+// passes 6.95 -> 6.5 ms; one 1080p view 282.2 -> 279.0 us a frame).
+__device__ __forceinline__ float clamp_nan(float x, float lo, float hi) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(lo));
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(r), "f"(hi));
+    return r;
+}
+
 // Exact floor(log2(m)) clamped to [0, levels-1]; m <= 0 or NaN -> 0,
 // +inf -> levels-1.
 __device__ __forceinline__ int hiz_level(float m, uint32_t levels) {
@@ -30,6 +42,19 @@ __device__ __forceinline__ int hiz_level(float m, uint32_t levels) {
     if (isinf(m)) return top;
     int e = (int)((__float_as_uint(m) >> 23) & 0xffu) - 127;  // subnormals give < 0 -> 0
     return e < 0 ? 0 : (e > top ? top : e);
+}
+
+// Whether every texel of [a0, a1] x [b0, b1] (at most 4 x 4, or empty) is >= z
+// (or NaN): a row's texels, the last one repeated, are in flight together.
+__device__ __forceinline__ bool texels_occlude(const float* img, uint32_t pitch, int a0, int a1, int b0, int b1, float z) {
+    if (a1 < a0) return true;
+    const int x1 = min(a0 + 1, a1), x2 = min(a0 + 2, a1);
+    for (int y = b0; y <= b1; ++y) {
+        const float* row = img + (size_t)y * pitch;
+        const float t0 = __ldg(row + a0), t1 = __ldg(row + x1), t2 = __ldg(row + x2), t3 = __ldg(row + a1);
+        if (t0 < z || t1 < z || t2 < z || t3 < z) return false;
+    }
+    return true;
 }
 
 // The fine occlusion addition (VKGV_CULL_OCCLUSION_FINE): every pyramid
@@ -54,19 +79,16 @@ __device__ __forceinline__ bool fine_occluded(const float* pyr, const uint32_t* 
     i1 = min(max(i1, 0), pw - 1);
     j0 = min(max(j0, 0), ph - 1);
     j1 = min(max(j1, 0), ph - 1);
-    for (int l = 0; l <= top; ++l) {
-        const int a0 = i0 >> l, a1 = i1 >> l, b0 = j0 >> l, b1 = j1 >> l;
-        if (a1 - a0 > 3 || b1 - b0 > 3) continue;
-        const uint32_t mw = mip_dim(pw0, (uint32_t)l);
-        const float* img = pyr + mips[l];
-        for (int y = b0; y <= b1; ++y)
-            for (int x = a0; x <= a1; ++x)
-                if (__ldg(img + (size_t)y * mw + x) < mx2) return false;
-        *foot = ((uint32_t)l << 28) | ((uint32_t)a0 << 16) | ((uint32_t)b0 << 4) | ((uint32_t)(a1 - a0) << 2) |
-                (uint32_t)(b1 - b0);
-        return true;
-    }
-    return false;
+    // the first level that holds the box: no level below the one where the
+    // wider range shifts to 3 or less does
+    const uint32_t wide = (uint32_t)max(max(i1 - i0, j1 - j0), 0);
+    int l = 32 - __clz((int)(wide >> 2));
+    if ((i1 >> l) - (i0 >> l) > 3 || (j1 >> l) - (j0 >> l) > 3) ++l;
+    if (l > top) return false;
+    const int a0 = i0 >> l, a1 = i1 >> l, b0 = j0 >> l, b1 = j1 >> l;
+    *foot = ((uint32_t)l << 28) | ((uint32_t)a0 << 16) | ((uint32_t)b0 << 4) | ((uint32_t)(a1 - a0) << 2) |
+            (uint32_t)(b1 - b0);
+    return texels_occlude(pyr + mips[l], mip_dim(pw0, (uint32_t)l), a0, a1, b0, b1, mx2);
 }
 
 // Repeats a fine footprint (the low word of a fine key) on a pyramid of the
@@ -76,11 +98,7 @@ __device__ __forceinline__ bool footprint_occluded(uint32_t foot, float mx2, con
     const uint32_t l = foot >> 28, a0 = (foot >> 16) & 0xfffu, b0 = (foot >> 4) & 0xfffu;
     const uint32_t a1 = a0 + ((foot >> 2) & 3u), b1 = b0 + (foot & 3u);
     const uint32_t mw = mip_dim(pw0, l);
-    const float* img = pyr + mips[l];
-    for (uint32_t y = b0; y <= b1; ++y)
-        for (uint32_t x = a0; x <= a1; ++x)
-            if (__ldg(img + (size_t)y * mw + x) < mx2) return false;
-    return true;
+    return texels_occlude(pyr + mips[l], mw, (int)a0, (int)a1, (int)b0, (int)b1, mx2);
 }
 
 // A meshlet's cone: two 16-byte loads where the array allows them.
@@ -177,14 +195,16 @@ __device__ __forceinline__ CullResult cull_one(const SceneArgs& S, const DeviceV
     // frustum and cone tests in pass 1 with the same planes and eye, and
     // would pass them again bit for bit, so only its occlusion is re-tested.
     if ((flags & VKGV_CULL_FRUSTUM) && !retest) {
+        bool outside = false;  // nearly all draws of a warp pass all planes: no branch per plane
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
             const float4 plane = frustum[i];
             const float p0 = plane.x, p1 = plane.y, p2 = plane.z, p3 = plane.w;
             float radius = fadd(fadd(fmul(we[0], fabsf(p0)), fmul(we[1], fabsf(p1))), fmul(we[2], fabsf(p2)));
             float distance = fsub(fadd(fadd(fmul(p0, wc4[0]), fmul(p1, wc4[1])), fmul(p2, wc4[2])), p3);
-            if (-radius > distance) return res;
+            outside |= -radius > distance;
         }
+        if (outside) return res;
     }
     // Meshlet normal-cone backface test (an addition; conservative with
     // respect to the per-triangle test of visbuffer.mesh.glsl:86-101, which
@@ -238,7 +258,7 @@ __device__ __forceinline__ CullResult cull_one(const SceneArgs& S, const DeviceV
                 for (int c = 0; c < 2; ++c) rows[j][a][b][c] = fadd(fadd(xy, mz[c]), m3);
             }
     }
-    float mn0 = 1.0f, mn1 = 1.0f, mn2 = 1.0f, mx0 = -1.0f, mx1 = -1.0f, mx2 = -1.0f;
+    float mn0 = 1.0f, mn1 = 1.0f, mx0 = -1.0f, mx1 = -1.0f, mx2 = -1.0f;
     bool all_front = true;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -249,18 +269,18 @@ __device__ __forceinline__ CullResult cull_one(const SceneArgs& S, const DeviceV
         // clip.xyz / clip.w as one correctly rounded reciprocal of w and three
         // products (within GLSL's 2.5 ulp for a division)
         const float rw = __frcp_rn(clip[3]);
-        float ndx = gclamp(fmul(clip[0], rw), -1.0f, 1.0f);
-        float ndy = gclamp(fmul(clip[1], rw), -1.0f, 1.0f);
-        float qx = fadd(fmul(ndx, 0.5f), 0.5f), qy = fadd(fmul(ndy, 0.5f), 0.5f);
-        float qz = fmul(clip[2], rw);
-        mn0 = gmin(mn0, qx);
-        mn1 = gmin(mn1, qy);
-        mn2 = gmin(mn2, qz);
-        mx0 = gmax(mx0, qx);
-        mx1 = gmax(mx1, qy);
-        mx2 = gmax(mx2, qz);
+        const float ndx = clamp_nan(fmul(clip[0], rw), -1.0f, 1.0f);
+        const float ndy = clamp_nan(fmul(clip[1], rw), -1.0f, 1.0f);
+        const float qx = fadd(fmul(ndx, 0.5f), 0.5f), qy = fadd(fmul(ndy, 0.5f), 0.5f);
+        // the bounds start as numbers, so a NaN corner leaves them (gmin and
+        // gmax keep their first argument then); of two zeros of mx2 either
+        // sign compares and is stored alike
+        mn0 = fminf(mn0, qx);
+        mn1 = fminf(mn1, qy);
+        mx0 = fmaxf(mx0, qx);
+        mx1 = fmaxf(mx1, qy);
+        mx2 = fmaxf(mx2, fmul(clip[2], rw));
     }
-    (void)mn2;
     // HiZ lookup (visbuffer.task.glsl:57-64)
     float width = fmul(fsub(mx0, mn0), (float)pw0);
     float height = fmul(fsub(mx1, mn1), (float)ph0);
@@ -360,23 +380,26 @@ __global__ void __launch_bounds__(256, 5) k_cull(SceneArgs S, const DeviceView* 
         s_mips[threadIdx.x - 96] = (uint32_t)mip_offset(first ? V.prev_w0 : V.w >> 1, first ? V.prev_h0 : V.h >> 1,
                                                         threadIdx.x - 96);
     }
-    if (threadIdx.x == 32) {
-        // the eye of the raster view-projection, for the cone test
+    if (threadIdx.x == 32) s_eye_ok = 0;
+    if (threadIdx.x == 32 && pass == 1) {
+        // the eye of the raster view-projection, for the cone test (which
+        // pass 2 does not repeat)
         float vp[16];
 #pragma unroll
         for (int k = 0; k < 16; ++k) vp[k] = cam->view_projection[k];
         s_eye_ok = (flags & VKGV_CULL_CONE) && S.cone_table && eye_from_vp(vp, s_eye);
     }
-    if (threadIdx.x == 64) {
+    if (threadIdx.x >= 64 && threadIdx.x < 96) {
         // Pass 2 can repeat the pass-1 lookups when the occlusion camera and
         // the pyramid's shape are unchanged (a static camera): the same box
         // projects to the same footprint.
-        int same = pass == 2 && V.reject_samples != nullptr && V.prev_pyr != nullptr && V.prev_levels != 0 &&
-                   V.prev_w0 == (V.w >> 1) && V.prev_h0 == (V.h >> 1) && V.prev_levels == V.pyr_levels;
-        for (int k = 0; same && k < 16; ++k)
-            same = __float_as_uint(cam->prev_occlusion_view_projection[k]) ==
-                   __float_as_uint(cam->occlusion_view_projection[k]);
-        s_same = same;
+        const uint32_t k = threadIdx.x & 15u;
+        const bool same = pass == 2 && V.reject_samples != nullptr && V.prev_pyr != nullptr && V.prev_levels != 0 &&
+                          V.prev_w0 == (V.w >> 1) && V.prev_h0 == (V.h >> 1) && V.prev_levels == V.pyr_levels &&
+                          __float_as_uint(cam->prev_occlusion_view_projection[k]) ==
+                              __float_as_uint(cam->occlusion_view_projection[k]);
+        const bool all = __all_sync(0xffffffffu, same);
+        if (threadIdx.x == 64) s_same = all;
     }
     __syncthreads();
     const float* eye = s_eye_ok ? s_eye : nullptr;
