@@ -248,6 +248,9 @@ int build_views(vkgv_ctx* ctx, const vkgv_scene* scene, const vkgv_view* views, 
         d.cam = reinterpret_cast<const vkgv_camera*>(v.camera_buffer);
         d.w = v.width;
         d.h = v.height;
+        d.inv_w = 1.0f / (float)v.width;
+        d.inv_h = 1.0f / (float)v.height;
+        d.div_w = v.width > 1 ? (uint32_t)((1ull << 32) / v.width) : 0xFFFFFFFFu;
         d.prev_pyr = reinterpret_cast<const float*>(v.prev_pyramid.data);
         d.prev_w0 = v.prev_pyramid.width;
         d.prev_h0 = v.prev_pyramid.height;

@@ -67,6 +67,9 @@ struct DeviceView {
     // box again when the occlusion camera and pyramid shape are unchanged;
     // null: pass 2 recomputes
     unsigned long long* reject_samples;
+    float inv_w, inv_h;         // 1 / w and 1 / h, correctly rounded
+    uint32_t div_w;             // floor(2^32 / w) (w = 1: 2^32 - 1), for pixel_xy
+    uint32_t _pad2;
 };
 
 struct SceneArgs {
@@ -101,6 +104,23 @@ __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
+
+// a / b for whole and half pixel coordinates a < b <= 8192 and inv = 1 / b
+// correctly rounded: a product and one residual correction give the IEEE
+// quotient (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990; equal for every such a and b).
+__device__ __forceinline__ float div_pixel(float a, float b, float inv) {
+    const float q = fmul(a, inv);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), inv, q);
+}
+
+// x = p % w, y = p / w for p < 2^32 by the precomputed floor(2^32 / w): the
+// product's high word is the quotient or one less.
+__device__ __forceinline__ void pixel_xy(uint32_t p, uint32_t w, uint32_t div_w, uint32_t& x, uint32_t& y) {
+    y = __umulhi(p, div_w);
+    x = p - y * w;
+    if (x >= w) x -= w, ++y;
+}
 
 // GLSL 4.60 min/max/clamp definitions.
 __device__ __forceinline__ float gmin(float x, float y) { return y < x ? y : x; }
