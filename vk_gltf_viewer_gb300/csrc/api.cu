@@ -196,8 +196,7 @@ struct Prepared {
     SceneArgs S;
     uint32_t max_w = 0, max_h = 0;
     uint64_t max_px = 0;
-    uint32_t hiz_tx = 1, hiz_ty = 1;  // single-pass HiZ grid (max over views)
-    uint32_t hiz_tail = 0;            // its tail's shared-memory floats (max over views)
+    HizShape hiz;                     // HiZ launch shape over the views
     float* tdets = nullptr;           // node tables filled by the clear (whole frames only)
     float* mvps = nullptr;
 };
@@ -278,13 +277,7 @@ int build_views(vkgv_ctx* ctx, const vkgv_scene* scene, const vkgv_view* views, 
         d.counters = ctx->counters + kGlobalCounters + kCountersPerView * i;
         P.max_w = std::max(P.max_w, v.width);
         P.max_h = std::max(P.max_h, v.height);
-        if (v.pyramid.levels) {
-            uint32_t tx = 1, ty = 1;
-            hiz_tiles(v.width, v.height, v.pyramid.levels, &tx, &ty);
-            P.hiz_tx = std::max(P.hiz_tx, tx);
-            P.hiz_ty = std::max(P.hiz_ty, ty);
-            P.hiz_tail = std::max(P.hiz_tail, hiz_tail_floats(v.width, v.height, v.pyramid.levels));
-        }
+        if (v.pyramid.levels) hiz_add_view(P.hiz, v.width, v.height, v.pyramid.levels);
         P.max_px = std::max<uint64_t>(P.max_px, (uint64_t)v.width * v.height);
     }
     return VKGV_OK;
@@ -334,7 +327,7 @@ void record_frame(vkgv_ctx* ctx, const Prepared& P, const DeviceView* dv, uint32
                   zones ? zones[3] : nullptr);
     zone(4);
     const bool two = (flags & VKGV_CULL_TWO_PASS) && (flags & VKGV_CULL_OCCLUSION);
-    if (two) launch_hiz(dv, n, P.hiz_tx, P.hiz_ty, P.hiz_tail, ctx->status, stream);
+    if (two) launch_hiz(dv, n, P.hiz, ctx->status, stream);
     zone(5);
     if (two) launch_cull(P.S, dv, n, flags, 2, ctx->status, ctx->sm_count, stream);
     zone(6);
@@ -355,12 +348,12 @@ void record_frame(vkgv_ctx* ctx, const Prepared& P, const DeviceView* dv, uint32
         // depth_id: the reduce runs on a side stream beside the resolve
         cudaEventRecord(ctx->fork_ev, stream);
         cudaStreamWaitEvent(ctx->side_stream, ctx->fork_ev, 0);
-        launch_hiz(dv, n, P.hiz_tx, P.hiz_ty, P.hiz_tail, ctx->status, ctx->side_stream);
+        launch_hiz(dv, n, P.hiz, ctx->status, ctx->side_stream);
         cudaEventRecord(ctx->join_ev, ctx->side_stream);
         launch_resolve(P.S, dv, n, P.max_w, P.max_h, flags, ctx->counters + 4, ctx->sm_count, stream);
         cudaStreamWaitEvent(stream, ctx->join_ev, 0);
     } else {
-        if (pyramid) launch_hiz(dv, n, P.hiz_tx, P.hiz_ty, P.hiz_tail, ctx->status, stream);
+        if (pyramid) launch_hiz(dv, n, P.hiz, ctx->status, stream);
         zone(9);
         if (resolve) launch_resolve(P.S, dv, n, P.max_w, P.max_h, flags, ctx->counters + 4, ctx->sm_count, stream);
     }
@@ -665,7 +658,7 @@ int vkgv_hiz_reduce(vkgv_ctx* ctx, const vkgv_view* view, void* stream_) {
     if (rc) return rc;
     rc = commit_views(ctx, slot, 1, stream);
     if (rc) return rc;
-    launch_hiz(dv, 1, P.hiz_tx, P.hiz_ty, P.hiz_tail, ctx->status, stream);
+    launch_hiz(dv, 1, P.hiz, ctx->status, stream);
     rc = check_launch(ctx);
     if (rc) return rc;
     return close_slot(ctx, slot, stream);

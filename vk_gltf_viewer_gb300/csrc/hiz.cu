@@ -106,13 +106,27 @@ __device__ __forceinline__ float reduce_texel(int x, int y, uint32_t dw, uint32_
     return r;
 }
 
+// FIRST: the levels over the depth image (and, unless hiz_second, all of
+// them).  Otherwise the levels over level 4, which take the place of the depth
+// image: level 4 + i of a view is (w >> 4) >> i wide, so that the reduction is
+// the same one on a smaller view.
+template <bool FIRST>
 __global__ void __launch_bounds__(kThreads, 5) k_hiz(const DeviceView* __restrict__ views, uint32_t* status,
                                                   uint32_t tail) {
     pdl_begin();
     const DeviceView& V = views[blockIdx.z];
     if (!V.pyr || V.pyr_levels == 0) return;
-    const uint32_t w = V.w, h = V.h, L = V.pyr_levels;
+    const bool second = hiz_second(V.w, V.h, V.pyr_levels);
+    if (!FIRST && !second) return;
+    constexpr uint32_t kSkip = FIRST ? 0u : (uint32_t)kHizTileLevels;
+    const uint32_t w = V.w >> kSkip, h = V.h >> kSkip, L = V.pyr_levels - kSkip;
     const uint32_t w0 = w >> 1, h0 = h >> 1;
+    float* const pyr = V.pyr + mip_offset(V.w >> 1, V.h >> 1, kSkip);
+    const float* const level4 = FIRST ? nullptr : V.pyr + mip_offset(V.w >> 1, V.h >> 1, kSkip - 1);
+    // texel (x, y) of the image under level 1
+    auto source = [&](int x, int y) {
+        return FIRST ? depth_at(V.depth_id, w, x, y) : __ldcg(level4 + (size_t)y * w + x);
+    };
     const int Kp = hiz_tile_levels(w, h, L);
     uint32_t ntx = 1, nty = 1;
     hiz_tiles(w, h, L, &ntx, &nty);
@@ -156,13 +170,13 @@ __global__ void __launch_bounds__(kThreads, 5) k_hiz(const DeviceView* __restric
             const uint32_t dw = w >> j, dh = h >> j;
             const uint32_t t = (uint32_t)hiz_tile_edge(j, Kp);
             const Range OX = owned(bx, t, dw), OY = owned(by, t, dh);
-            float* dst = V.pyr + mip_offset(w0, h0, (uint32_t)(j - 1));
+            float* dst = pyr + mip_offset(w0, h0, (uint32_t)(j - 1));
             float* here = lvl[j];
             const float* below = lvl[j - 1];
             const Range BX = j > 1 ? rx[j - 1] : Range{0, 0};
             const Range BY = j > 1 ? ry[j - 1] : Range{0, 0};
             const int bw = BX.hi - BX.lo + 1;
-            if (j == 1 && w == 2 * dw && h == 2 * dh) {
+            if (FIRST && j == 1 && w == 2 * dw && h == 2 * dh) {
                 // Level 1 over the depth image, 2x2 blocks with one 16-byte
                 // load per row (depth_id is 16-byte aligned and w is even).
                 // Batches of four texels per thread: all eight loads are in
@@ -200,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_hiz(const DeviceView* __restric
                 const int x = X.lo + i % rw, y = Y.lo + i / rw;
                 float r;
                 if (j == 1) {
-                    r = reduce_texel(x, y, dw, dh, w, h, [&](int sx, int sy) { return depth_at(V.depth_id, w, sx, sy); });
+                    r = reduce_texel(x, y, dw, dh, w, h, source);
                 } else {
                     r = reduce_texel(x, y, dw, dh, w >> (j - 1), h >> (j - 1),
                                      [&](int sx, int sy) { return below[(sy - BY.lo) * bw + (sx - BX.lo)]; });
@@ -211,6 +225,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_hiz(const DeviceView* __restric
             __syncthreads();
         }
     }
+    if (FIRST && second) return;  // the second launch reduces the rest
     // The last CTA of this view finishes levels Kp+1..L.
     __threadfence();
     __syncthreads();
@@ -261,7 +276,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_hiz(const DeviceView* __restric
         float* lv = smem;
         const uint64_t base = mip_offset(w0, h0, (uint32_t)Kp);  // level Kp+1
         {
-            const float* src = V.pyr + (base - (uint64_t)top_w * top_h);  // the top tiled mip
+            const float* src = pyr + (base - (uint64_t)top_w * top_h);  // the top tiled mip
             const uint32_t dw = w >> (Kp + 1), sw = top_w, n = next_px;
             for (uint32_t i0 = threadIdx.x; i0 < n; i0 += kTailBatch * kThreads) {
                 float t[kTailBatch][4];
@@ -324,7 +339,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_hiz(const DeviceView* __restric
             __syncthreads();
         }
         // every tail level out in one coalesced pass
-        float* dst = V.pyr + base;
+        float* dst = pyr + base;
         for (uint32_t i = threadIdx.x; i < so + sz; i += kThreads) dst[i] = lv[i];
         first_zero = Lv + 1;
     }
@@ -332,17 +347,17 @@ __global__ void __launch_bounds__(kThreads, 5) k_hiz(const DeviceView* __restric
     for (uint32_t j = first_zero; j <= L; ++j) {
         const uint32_t dw = w >> j, dh = h >> j;
         const uint32_t mw = mip_dim(w0, j - 1), mh = mip_dim(h0, j - 1);
-        float* dst = V.pyr + mip_offset(w0, h0, j - 1);
+        float* dst = pyr + mip_offset(w0, h0, j - 1);
         if (dw == 0 || dh == 0) {
             for (uint32_t i = threadIdx.x; i < mw * mh; i += blockDim.x) dst[i] = 0.0f;
         } else {
             const uint32_t sw = j == 1 ? w : mip_dim(w0, j - 2), sh = j == 1 ? h : mip_dim(h0, j - 2);
-            const float* src = j == 1 ? nullptr : V.pyr + mip_offset(w0, h0, j - 2);
+            const float* src = j == 1 ? nullptr : pyr + mip_offset(w0, h0, j - 2);
             for (uint32_t i = threadIdx.x; i < dw * dh; i += blockDim.x) {
                 const int x = (int)(i % dw), y = (int)(i / dw);
                 float r;
                 if (j == 1)
-                    r = reduce_texel(x, y, dw, dh, sw, sh, [&](int sx, int sy) { return depth_at(V.depth_id, w, sx, sy); });
+                    r = reduce_texel(x, y, dw, dh, sw, sh, source);
                 else
                     r = reduce_texel(x, y, dw, dh, sw, sh,
                                      [&](int sx, int sy) { return __ldcg(src + (size_t)sy * sw + sx); });
@@ -356,8 +371,11 @@ __global__ void __launch_bounds__(kThreads, 5) k_hiz(const DeviceView* __restric
 
 }  // namespace
 
-uint32_t hiz_tail_floats(uint32_t w, uint32_t h, uint32_t levels) {
-    // the levels above the tiled ones that have no zero dimension
+namespace {
+
+// Shared-memory floats of the tail: the levels above the tiled ones that have
+// no zero dimension.
+uint32_t tail_floats(uint32_t w, uint32_t h, uint32_t levels) {
     const int top = hiz_tile_levels(w, h, levels);
     uint32_t sum = 0;
     for (uint32_t j = (uint32_t)top + 1; top > 0 && j <= levels && (w >> j) != 0 && (h >> j) != 0; ++j)
@@ -365,8 +383,9 @@ uint32_t hiz_tail_floats(uint32_t w, uint32_t h, uint32_t levels) {
     return sum;
 }
 
-void launch_hiz(const DeviceView* views, uint32_t nviews, uint32_t tiles_x, uint32_t tiles_y, uint32_t tail,
-                uint32_t* status, cudaStream_t stream) {
+template <bool FIRST>
+void launch_pass(const DeviceView* views, uint32_t nviews, uint32_t tiles_x, uint32_t tiles_y, uint32_t tail,
+                 uint32_t* status, cudaStream_t stream) {
     // The dynamic shared-memory limit is a per-device function attribute:
     // set it once for each device a launch runs on (setting it twice is
     // harmless, so concurrent first launches need no lock).
@@ -375,14 +394,42 @@ void launch_hiz(const DeviceView* views, uint32_t nviews, uint32_t tiles_x, uint
     cudaGetDevice(&dev);
     const uint64_t bit = dev < 64 ? (1ull << dev) : 0ull;
     if (!bit || !(attr_devices.load(std::memory_order_acquire) & bit)) {
-        cudaFuncSetAttribute(k_hiz, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMax * (int)sizeof(float));
+        cudaFuncSetAttribute(k_hiz<FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMax * (int)sizeof(float));
         attr_devices.fetch_or(bit, std::memory_order_release);
     }
     // the tail works in shared memory when all of its levels fit
     if (tail > (uint32_t)kTailMax) tail = 0;
     const uint32_t floats = tail > (uint32_t)kTileFloats ? tail : (uint32_t)kTileFloats;
     dim3 grid(tiles_x ? tiles_x : 1, tiles_y ? tiles_y : 1, nviews);
-    launch_pdl(k_hiz, grid, dim3(kThreads), floats * sizeof(float), stream, views, status, tail);
+    launch_pdl(k_hiz<FIRST>, grid, dim3(kThreads), floats * sizeof(float), stream, views, status, tail);
+}
+
+}  // namespace
+
+void hiz_add_view(HizShape& shape, uint32_t w, uint32_t h, uint32_t levels) {
+    auto widen = [](uint32_t& tx, uint32_t& ty, uint32_t vw, uint32_t vh, uint32_t vl) {
+        uint32_t x = 1, y = 1;
+        hiz_tiles(vw, vh, vl, &x, &y);
+        tx = x > tx ? x : tx;
+        ty = y > ty ? y : ty;
+    };
+    widen(shape.tiles_x, shape.tiles_y, w, h, levels);
+    if (hiz_second(w, h, levels)) {
+        w >>= kHizTileLevels, h >>= kHizTileLevels, levels -= kHizTileLevels;
+        widen(shape.tiles_x2, shape.tiles_y2, w, h, levels);
+        const uint32_t t = tail_floats(w, h, levels);
+        shape.tail2 = t > shape.tail2 ? t : shape.tail2;
+    } else {
+        const uint32_t t = tail_floats(w, h, levels);
+        shape.tail = t > shape.tail ? t : shape.tail;
+    }
+}
+
+void launch_hiz(const DeviceView* views, uint32_t nviews, const HizShape& shape, uint32_t* status,
+                cudaStream_t stream) {
+    launch_pass<true>(views, nviews, shape.tiles_x, shape.tiles_y, shape.tail, status, stream);
+    if (shape.tiles_x2)
+        launch_pass<false>(views, nviews, shape.tiles_x2, shape.tiles_y2, shape.tail2, status, stream);
 }
 
 }  // namespace vkgv
