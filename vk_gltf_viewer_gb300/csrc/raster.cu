@@ -39,11 +39,16 @@ __device__ __forceinline__ bool outside_guard(const float4& v) {
     return v.x < -g || v.x > g || v.y < -g || v.y > g;
 }
 
+// What a warp's raster needs of its current view (in shared memory: fewer
+// live registers), and of the launch (one per CTA).
 struct RasterCtx {
     unsigned long long* depth;
     uint32_t w, h;
     float hw, hh;
     uint32_t view;
+};
+
+struct RasterQueue {
     BigTri* big;
     uint32_t* big_count;
     uint32_t big_cap;
@@ -107,7 +112,7 @@ struct BinJob {
     float z0, pa, pb;         // depth plane
     uint32_t id;
     int32_t px0, py0, px1, py1;  // clamped pixel bounding box
-    uint32_t n;               // rectangles of c.chunk x c.chunk pixels
+    uint32_t n;               // rectangles of Q.chunk x Q.chunk pixels
 };
 // A clipped triangle fans into at most 10 triangles.
 constexpr uint32_t kMaxJobs = 10;
@@ -116,11 +121,11 @@ struct JobList {
     uint32_t count;
 };
 
-// The rectangles of one job, queued at c.big[at, at + n) (past the queue's
+// The rectangles of one job, queued at Q.big[at, at + n) (past the queue's
 // capacity they are drawn in place and the overflow is reported).
-__device__ void queue_job(const BinJob& j, uint32_t at, const RasterCtx& c) {
-    const int32_t cs = (int32_t)c.chunk;
-    const uint32_t ncx = (uint32_t)(j.px1 - j.px0 + cs) >> c.chunk_log2;
+__device__ void queue_job(const BinJob& j, uint32_t at, const RasterCtx& c, const RasterQueue& Q) {
+    const int32_t cs = (int32_t)Q.chunk;
+    const uint32_t ncx = (uint32_t)(j.px1 - j.px0 + cs) >> Q.chunk_log2;
     uint32_t flags = kBigNarrow;
     int32_t bias[3];
 #pragma unroll
@@ -135,7 +140,7 @@ __device__ void queue_job(const BinJob& j, uint32_t at, const RasterCtx& c) {
     for (uint32_t i = 0; i < j.n; ++i, ++at, ++cx, qx0 += cs) {
         if (cx == ncx) cx = 0, qx0 = j.px0, qy0 += cs;
         const int32_t qx1 = min(j.px1, qx0 + cs - 1), qy1 = min(j.py1, qy0 + cs - 1);
-        if (at < c.big_cap) {
+        if (at < Q.big_cap) {
             BigTri t;
             t.x[0] = j.x[0], t.x[1] = j.x[1], t.x[2] = j.x[2];
             t.y[0] = j.y[0], t.y[1] = j.y[1], t.y[2] = j.y[2];
@@ -144,9 +149,9 @@ __device__ void queue_job(const BinJob& j, uint32_t at, const RasterCtx& c) {
             t.px0 = (uint16_t)qx0, t.py0 = (uint16_t)qy0, t.px1 = (uint16_t)qx1, t.py1 = (uint16_t)qy1;
             t.view = c.view;
             t.flags = flags;
-            c.big[at] = t;
+            Q.big[at] = t;
         } else {
-            report(c.status, kStatusQueueOverflow, at);
+            report(Q.status, kStatusQueueOverflow, at);
             raster_rect(j.x, j.y, bias, j.z0, j.pa, j.pb, j.id, qx0, qy0, qx1, qy1, c.depth, c.w);
         }
     }
@@ -154,7 +159,7 @@ __device__ void queue_job(const BinJob& j, uint32_t at, const RasterCtx& c) {
 
 // Queues the jobs of every lane (the whole warp, converged): an exclusive
 // scan of the lanes' rectangle counts, one atomic on the queue counter.
-__device__ void flush_jobs(JobList& jobs, const RasterCtx& c, int lane) {
+__device__ void flush_jobs(JobList& jobs, const RasterCtx& c, const RasterQueue& Q, int lane) {
     uint32_t mine = 0;
     for (uint32_t i = 0; i < jobs.count; ++i) mine += jobs.job[i].n;
     uint32_t incl = mine;
@@ -169,10 +174,10 @@ __device__ void flush_jobs(JobList& jobs, const RasterCtx& c, int lane) {
         return;
     }
     uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(c.big_count, total);
+    if (lane == 0) base = atomicAdd(Q.big_count, total);
     base = __shfl_sync(0xffffffffu, base, 0) + (incl - mine);
     for (uint32_t i = 0; i < jobs.count; ++i) {
-        queue_job(jobs.job[i], base, c);
+        queue_job(jobs.job[i], base, c, Q);
         base += jobs.job[i].n;
     }
     jobs.count = 0;
@@ -182,7 +187,7 @@ __device__ void flush_jobs(JobList& jobs, const RasterCtx& c, int lane) {
 // raster; a triangle to bin becomes a job in `jobs` (queued directly when
 // the list is full).
 __device__ __noinline__ void setup_and_raster(int32_t X0, int32_t Y0, float Z0, int32_t X1, int32_t Y1, float Z1, int32_t X2,
-                                 int32_t Y2, float Z2, uint32_t id, const RasterCtx& c, JobList& jobs) {
+                                 int32_t Y2, float Z2, uint32_t id, const RasterCtx& c, const RasterQueue& Q, JobList& jobs) {
     int64_t A = (int64_t)(X1 - X0) * (Y2 - Y0) - (int64_t)(Y1 - Y0) * (X2 - X0);
     if (A == 0) return;
     if (A < 0) {
@@ -218,11 +223,11 @@ __device__ __noinline__ void setup_and_raster(int32_t X0, int32_t Y0, float Z0, 
     const float pa = fmul(fsub(fmul(dz1, dy2), fmul(dz2, dy1)), ra);
     const float pb = fmul(fsub(fmul(dz2, dx1), fmul(dz1, dx2)), ra);
     const int64_t bw = px1 - px0 + 1, bh = py1 - py0 + 1;
-    if (bw * bh <= (int64_t)c.small_area) {
+    if (bw * bh <= (int64_t)Q.small_area) {
         raster_rect(X, Y, bias, Z0, pa, pb, id, (int)px0, (int)py0, (int)px1, (int)py1, c.depth, c.w);
         return;
     }
-    const uint32_t ncx = (uint32_t)(bw + c.chunk - 1) >> c.chunk_log2, ncy = (uint32_t)(bh + c.chunk - 1) >> c.chunk_log2;
+    const uint32_t ncx = (uint32_t)(bw + Q.chunk - 1) >> Q.chunk_log2, ncy = (uint32_t)(bh + Q.chunk - 1) >> Q.chunk_log2;
     BinJob j;
     j.x[0] = X0, j.x[1] = X1, j.x[2] = X2;
     j.y[0] = Y0, j.y[1] = Y1, j.y[2] = Y2;
@@ -233,7 +238,7 @@ __device__ __noinline__ void setup_and_raster(int32_t X0, int32_t Y0, float Z0, 
     if (jobs.count < kMaxJobs) {
         jobs.job[jobs.count++] = j;
     } else {
-        queue_job(j, atomicAdd(c.big_count, j.n), c);
+        queue_job(j, atomicAdd(Q.big_count, j.n), c, Q);
     }
 }
 
@@ -288,7 +293,7 @@ __device__ int clip_poly(const float4* in, int n, float4* out, int plane) {
 
 // Slow path: homogeneous clipping (near/far, then guard band) and a fan.
 __device__ __noinline__ void raster_clipped(float4 v0, float4 v1, float4 v2, bool clipz, uint32_t id,
-                                            const RasterCtx& c, JobList& jobs) {
+                                            const RasterCtx& c, const RasterQueue& Q, JobList& jobs) {
     float4 bufa[12], bufb[12];
     bufa[0] = v0, bufa[1] = v1, bufa[2] = v2;
     float4* cur = bufa;
@@ -318,7 +323,7 @@ __device__ __noinline__ void raster_clipped(float4 v0, float4 v1, float4 v2, boo
     for (int k = 0; k < n; ++k)
         if (!snap(cur[k], c, X[k], Y[k], Z[k])) return;
     for (int k = 1; k + 1 < n; ++k)
-        setup_and_raster(X[0], Y[0], Z[0], X[k], Y[k], Z[k], X[k + 1], Y[k + 1], Z[k + 1], id, c, jobs);
+        setup_and_raster(X[0], Y[0], Z[0], X[k], Y[k], Z[k], X[k + 1], Y[k + 1], Z[k + 1], id, c, Q, jobs);
 }
 
 // Items a warp takes at once, at most (256-view torus grid 32.1 ms; 16: 32.4;
@@ -450,9 +455,9 @@ struct TriClass {
 template <bool SLOW>
 __device__ __forceinline__ int classify(uint32_t i0, uint32_t i1, uint32_t i2, uint32_t vc, const int2* sxy,
                                         const int2* szf, const float4* clip, bool double_sided, float tdet, const RasterCtx& c,
-                                        uint32_t d, TriClass& k) {
+                                        const RasterQueue& Q, uint32_t d, TriClass& k) {
     if (i0 >= vc || i1 >= vc || i2 >= vc) {
-        if (!SLOW) report(c.status, kStatusBadIndex, d);
+        if (!SLOW) report(Q.status, kStatusBadIndex, d);
         return kDrop;
     }
     k.q0 = sxy[i0], k.f0 = szf[i0];
@@ -477,7 +482,7 @@ __device__ __forceinline__ int classify(uint32_t i0, uint32_t i1, uint32_t i2, u
     const int64_t A = (int64_t)(q1.x - q0.x) * (q2.y - q0.y) - (int64_t)(q1.y - q0.y) * (q2.x - q0.x);
     if (A == 0) return kDrop;
     const bool small = maxx - minx < kSmallExtent && maxy - miny < kSmallExtent &&
-                       (uint32_t)((qx1 - qx0 + 1) * (qy1 - qy0 + 1)) <= c.small_area;
+                       (uint32_t)((qx1 - qx0 + 1) * (qy1 - qy0 + 1)) <= Q.small_area;
     return small ? kFast : kSlowSetup;
 }
 
@@ -549,8 +554,8 @@ __device__ __forceinline__ unsigned long long fragment(float pa, float pb, float
 // the larger ones are spread over the warp by a scan of their bbox areas.
 // xyw holds each vertex's clip x, y, w and snapped depth.
 __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, const int2* sxy, const float4* xyw,
-                                             bool double_sided, float tdet, uint32_t d, const RasterCtx& c,
-                                             TriRec* recs, uint32_t* starts, int lane) {
+                                             bool double_sided, float tdet, uint32_t d, const RasterCtx& c, const RasterQueue& Q,
+                                             TriRec* recs, uint16_t* starts, int lane) {
     uint32_t coop_area = 0;
     bool slow = false;
     TriRec rec;
@@ -573,7 +578,7 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
         const int32_t px0 = max((minx - 128 + 255) >> 8, 0), px1 = min((maxx - 128) >> 8, (int32_t)c.w - 1);
         const int32_t py0 = max((miny - 128 + 255) >> 8, 0), py1 = min((maxy - 128) >> 8, (int32_t)c.h - 1);
         const uint32_t bw = (uint32_t)(px1 - px0 + 1), bh = (uint32_t)(py1 - py0 + 1);
-        const bool live = !back && fits && A != 0 && bw * bh <= c.small_area;
+        const bool live = !back && fits && A != 0 && bw * bh <= Q.small_area;
         if (!back && !live) {
             const int64_t A64 = (int64_t)(q1.x - q0.x) * (q2.y - q0.y) - (int64_t)(q1.y - q0.y) * (q2.x - q0.x);
             slow = A64 != 0;
@@ -641,11 +646,11 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
     if (mm) {
         const int leader = __ffs(mm) - 1;
         uint32_t base = 0;
-        if (lane == leader) base = atomicAdd(c.big_count, (uint32_t)__popc(mm));
+        if (lane == leader) base = atomicAdd(Q.big_count, (uint32_t)__popc(mm));
         base = __shfl_sync(0xffffffffu, base, leader);
         if (coop_area > kQueueArea) {
             const uint32_t slot = base + (uint32_t)__popc(mm & ((1u << lane) - 1u));
-            if (slot < c.big_cap) {
+            if (slot < Q.big_cap) {
                 const uint32_t px0 = rec.origin & 0xFFFFu, py0 = rec.origin >> 16, bw = (rec.bits >> 10) & 127u;
                 BigTri t;
 #pragma unroll
@@ -659,10 +664,10 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
                 t.px1 = (uint16_t)(px0 + bw - 1u), t.py1 = (uint16_t)(py0 + coop_area / bw - 1u);
                 t.view = c.view;
                 t.flags = ((rec.bits >> 7) & 7u) | kBigNarrow;
-                c.big[slot] = t;
+                Q.big[slot] = t;
                 coop_area = 0;
             } else {
-                report(c.status, kStatusQueueOverflow, slot);
+                report(Q.status, kStatusQueueOverflow, slot);
             }
         }
         coop = __ballot_sync(0xffffffffu, coop_area != 0);
@@ -684,7 +689,7 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
     if (coop_area) {
         const uint32_t at = (uint32_t)__popc(coop & ((1u << lane) - 1u));
         recs[at] = rec;
-        starts[at] = start;
+        starts[at] = (uint16_t)start;  // below 32 * 64
     }
     __syncwarp();
     for (uint32_t p0 = 0; p0 < total; p0 += 32) {
@@ -728,15 +733,14 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
     __shared__ TriRec s_tri[WARPS][32];
     // the compacted candidate triangle indices (fast instance)
     __shared__ uint8_t s_ring[WARPS][128];
-    __shared__ uint32_t s_start[WARPS][32];
+    __shared__ uint16_t s_start[WARPS][32];
     __shared__ float s_mvp[WARPS][16];
     __shared__ float s_tdet[WARPS];
-    __shared__ float s_vp[WARPS][16];
     // exclusive prefix of the views' work counts: view v owns the global
     // work items [s_pre[v], s_pre[v + 1])
-    // (sized by the launch: with the flags sharing the records' memory, 20 KB a
-    // CTA instead of 25, which leaves more L1: the 1080p torus grid's frame
-    // 308.0 -> 305.6 us)
+    // (sized by the launch: 18 KB a CTA leave seven of them in 132 KB and the
+    // rest to the L1: the 1080p torus grid's frame 308.0 -> 305.6 us from 25 to
+    // 20 KB, 276.3 -> 274.3 us to 18)
     extern __shared__ uint32_t s_pre[];  // nviews + 1
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t nv = P.nviews;
@@ -746,7 +750,17 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
         view_work<SLOW>(P, P.views[v], l, n, f);
         s_pre[v + 1] = n;
     }
-    if (threadIdx.x == 0) s_pre[0] = 0;
+    __shared__ RasterQueue Q;
+    if (threadIdx.x == 0) {
+        s_pre[0] = 0;
+        Q.big = P.big;
+        Q.big_count = P.big_count;
+        Q.big_cap = P.big_cap;
+        Q.small_area = P.small_area;
+        Q.chunk = P.chunk;
+        Q.chunk_log2 = 31u - (uint32_t)__clz((int)P.chunk);
+        Q.status = P.status;
+    }
     __syncthreads();
     if (warp == 0) {
         // inclusive scan of s_pre[1..nv]: lane-contiguous segments, then a
@@ -785,26 +799,16 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
     uint32_t* sidx = s_idx[warp];
     const uint8_t* sidx8 = reinterpret_cast<const uint8_t*>(sidx);
     TriRec* recs = s_tri[warp];
-    uint32_t* starts = s_start[warp];
+    uint16_t* starts = s_start[warp];
     // Warps take runs of `grab` consecutive work items from one counter, so
     // views are drawn roughly in order (their depth buffers stay in L2) and
     // no warp idles while work is left.
     const uint32_t warps_total = gridDim.x * WARPS;
     const uint32_t grab = max(1u, min(kMaxRun, total / (warps_total * 8u)));
-    uint32_t cur_v = 0xffffffffu, cur_t = 0xffffffffu;  // view and node of s_vp / s_mvp
+    uint32_t cur_v = 0xffffffffu, cur_t = 0xffffffffu;  // view and node of s_mvp
     const DeviceView* Vp = P.views;
-    // the warp's raster context lives in shared memory (fewer live registers)
     __shared__ RasterCtx s_ctx[WARPS];
     RasterCtx& c = s_ctx[warp];
-    if (lane == 0) {
-        c.big = P.big;
-        c.big_count = P.big_count;
-        c.big_cap = P.big_cap;
-        c.small_area = P.small_area;
-        c.chunk = P.chunk;
-        c.chunk_log2 = 31u - (uint32_t)__clz((int)P.chunk);
-        c.status = P.status;
-    }
     // Per-meshlet headers of the current run, resolved one item per lane so
     // that the dependent loads (list entry -> draw -> primitive -> meshlet
     // record, material) of up to kMaxRun meshlets are in flight together instead
@@ -904,7 +908,6 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
                     c.hh = 0.5f * (float)Vp->h;
                     c.view = P.view_base + v;
                 }
-                if (lane < 16) s_vp[warp][lane] = Vp->cam->view_projection[lane];
                 __syncwarp();
             }
             const DeviceView& V = *Vp;
@@ -928,9 +931,10 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
             } else if (lane < 16) {
                 const int cc = lane >> 2, j = lane & 3;
                 const float4 mc = __ldg(reinterpret_cast<const float4*>(Mg) + cc);
-                s_mvp[warp][lane] = fadd(fadd(fadd(fmul(s_vp[warp][0 * 4 + j], mc.x), fmul(s_vp[warp][1 * 4 + j], mc.y)),
-                                              fmul(s_vp[warp][2 * 4 + j], mc.z)),
-                                         fmul(s_vp[warp][3 * 4 + j], mc.w));
+                const float* vp = V.cam->view_projection;
+                s_mvp[warp][lane] = fadd(fadd(fadd(fmul(vp[0 * 4 + j], mc.x), fmul(vp[1 * 4 + j], mc.y)),
+                                              fmul(vp[2 * 4 + j], mc.z)),
+                                         fmul(vp[3 * 4 + j], mc.w));
             } else if (lane == 16 && have_tdet) {
                 s_tdet[warp] = P.S.tdets[transform_index];
             } else if (lane == 16) {
@@ -1019,19 +1023,19 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
                     if (t < tc) {
                         TriClass k;
                         const uint32_t i0 = sidx8[3 * t], i1 = sidx8[3 * t + 1], i2 = sidx8[3 * t + 2];
-                        const int kind = classify<true>(i0, i1, i2, vc, sxy, szf, clip, double_sided, tdet, c, d, k);
+                        const int kind = classify<true>(i0, i1, i2, vc, sxy, szf, clip, double_sided, tdet, c, Q, d, k);
                         if (kind == kSlowClip) {
                             raster_clipped(clip[i0], clip[i1], clip[i2],
                                            ((uint32_t)(k.f0.y | k.f1.y | k.f2.y) & (OC_ZLO | OC_ZHI)) != 0,
-                                           (d << 7) | t, c, jobs);
+                                           (d << 7) | t, c, Q, jobs);
                         } else if (kind == kSlowSetup) {
                             setup_and_raster(k.q0.x, k.q0.y, __int_as_float(k.f0.x), k.q1.x, k.q1.y,
                                              __int_as_float(k.f1.x), k.q2.x, k.q2.y, __int_as_float(k.f2.x),
-                                             (d << 7) | t, c, jobs);
+                                             (d << 7) | t, c, Q, jobs);
                         }
                     }
                     __syncwarp();
-                    flush_jobs(jobs, c, lane);
+                    flush_jobs(jobs, c, Q, lane);
                 }
             } else {
                 // Pre-filter 32 triangles per round (a pixel centre in the
@@ -1064,7 +1068,7 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
                 __syncwarp();
                 for (uint32_t at = 0; at < pending; at += 32) {
                     const uint32_t ct = at + lane < pending ? ring[at + lane] : 0xffffffffu;
-                    any_slow |= raster_small(ct, sidx8, sxy, clip, double_sided, tdet, d, c, recs, starts, lane);
+                    any_slow |= raster_small(ct, sidx8, sxy, clip, double_sided, tdet, d, c, Q, recs, starts, lane);
                 }
             }
             if (!SLOW && __any_sync(0xffffffffu, any_slow) && lane == 0) {
