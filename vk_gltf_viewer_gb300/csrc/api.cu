@@ -823,6 +823,7 @@ int vkgv_world_create(vkgv_ctx* ctx, const vkgv_world_desc* desc, vkgv_world** o
     A.slot_count = P.slot_count;
     A.seg_count = P.seg_count;
     A.draw_count = (uint32_t)P.draw_count;
+    A.max_chain = P.max_chain;
     w->draw_count = P.draw_count;
     *out_world = w;
     return VKGV_OK;

@@ -165,6 +165,7 @@ struct WorldArgs {
     uint32_t seg_count;
     uint32_t draw_count;
     uint32_t tile_count;
+    uint32_t max_chain;             // nodes on the longest path
 };
 
 constexpr uint32_t kWorldTile = 1024;    // draws per k_world_draws block
@@ -181,13 +182,13 @@ struct WorldPlan {
     std::vector<uint32_t> seg_first;
     std::vector<uint2> seg_info;
     std::vector<uint32_t> tile_seg;
-    uint32_t node_count = 0, slot_count = 0, seg_count = 0;
+    uint32_t node_count = 0, slot_count = 0, seg_count = 0, max_chain = 0;
     uint64_t draw_count = 0;
 };
 
 // Validates a world description and walks its tree; returns a vkgv_status.
 int plan_world(const vkgv_world_desc& desc, WorldPlan& plan, std::string& err);
-// k_world_local + k_world_chain: transforms[16 * slot] at `time`.
+// transforms[16 * slot] at `time`.
 void launch_world_transforms(const WorldArgs& W, float time, float* transforms, cudaStream_t stream);
 // k_world_draws: the MeshletDraw list as 3 words per draw.
 void launch_world_draws(const WorldArgs& W, uint32_t* draws, uint32_t sm_count, cudaStream_t stream);

@@ -6,12 +6,14 @@
 // sampling every channel of every animation for every node, composing
 // parent * T * R * S, and copies the transforms (and, on a scene change, the
 // draw list) into mapped buffers.  Here the host walks the tree once
-// (plan_world) and each frame is two kernels:
-//   k_world_local  one thread per node: rest TRS, the node's channels in
-//                  application order, local matrix T * R * S;
-//   k_world_chain  one thread per transform slot: the product of the local
-//                  matrices from the root down its path, in the reference's
-//                  association order ((I * L_root) * ...) * L_node.
+// (plan_world) and each frame evaluates, per transform slot, the local matrices
+// T * R * S (rest TRS, the node's channels in application order) of its path
+// and their product from the root down in the reference's association order
+// ((I * L_root) * ...) * L_node:
+//   k_world_slots  a group of lanes per slot, one lane per node of the path,
+//                  then the product by shuffles;
+//   k_world_local, k_world_chain  deep or large trees (launch_world_transforms
+//                  has the line): one thread per node, then one per slot.
 // The draw list is k_world_draws: one block per tile of 1024 draws whose
 // first segment the plan holds, the tile's records staged in shared memory
 // and stored as 16-byte words.
@@ -173,10 +175,8 @@ __device__ void trs_matrix(const float t[3], const float q[4], const float s[3],
     m[12] = t[0], m[13] = t[1], m[14] = t[2], m[15] = 1.0f;
 }
 
-__global__ void __launch_bounds__(128) k_world_local(WorldArgs W, float time) {
-    pdl_begin();
-    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= W.node_count) return;
+// T * R * S of node n at `time`.
+__device__ __forceinline__ void local_matrix(const WorldArgs& W, uint32_t n, float time, float m[16]) {
     const float* r = W.rest + 10 * (size_t)n;
     float t[3] = {r[0], r[1], r[2]}, q[4] = {r[3], r[4], r[5], r[6]}, s[3] = {r[7], r[8], r[9]};
     // World::iterateNode (world.cpp:187-215): every channel that targets the
@@ -192,8 +192,51 @@ __global__ void __launch_bounds__(128) k_world_local(WorldArgs W, float time) {
         else
             s[0] = v[0], s[1] = v[1], s[2] = v[2];
     }
-    float m[16];
     trs_matrix(t, q, s, m);
+}
+
+// Bound by one chain of dependent loads (path -> channels -> sampler -> keys):
+// the nodes of a path take it side by side, where one launch for the nodes
+// and one for the products took it twice.  2,048 tori, two nodes a path:
+// 8.6 -> 6.7 us, with the draw list 15.9 -> 13.2 us.
+template <uint32_t G>
+__global__ void __launch_bounds__(128) k_world_slots(WorldArgs W, float time, float* __restrict__ transforms) {
+    pdl_begin();
+    const uint32_t slot = (blockIdx.x * blockDim.x + threadIdx.x) / G, r = threadIdx.x % G;
+    uint32_t first = 0, len = 0;
+    if (slot < W.slot_count) {
+        first = W.chain_offsets[slot];
+        len = W.chain_offsets[slot + 1] - first;
+    }
+    float L[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) L[i] = 0.0f;
+    if (r < len) local_matrix(W, W.chain_nodes[first + r], time, L);
+    float M[16] = {1.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f};
+#pragma unroll
+    for (uint32_t k = 0; k < G; ++k) {
+        float A[16], R[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) A[i] = __shfl_sync(0xffffffffu, L[i], (int)k, (int)G);
+        if (k < len) {
+            m4m(M, A, R);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) M[i] = R[i];
+        }
+    }
+    if (slot >= W.slot_count) return;
+    float4* out = reinterpret_cast<float4*>(transforms + 16 * (size_t)slot);
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k)
+        if (k % G == r) out[k] = make_float4(M[4 * k], M[4 * k + 1], M[4 * k + 2], M[4 * k + 3]);
+}
+
+__global__ void __launch_bounds__(128) k_world_local(WorldArgs W, float time) {
+    pdl_begin();
+    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= W.node_count) return;
+    float m[16];
+    local_matrix(W, n, time, m);
     float4* out = reinterpret_cast<float4*>(W.local + 16 * (size_t)n);
     for (int k = 0; k < 4; ++k) out[k] = make_float4(m[4 * k], m[4 * k + 1], m[4 * k + 2], m[4 * k + 3]);
 }
@@ -265,7 +308,33 @@ __global__ void __launch_bounds__(kWorldThreads) k_world_draws(WorldArgs W, uint
 
 }  // namespace
 
+namespace {
+
+template <uint32_t G>
+void launch_slots(const WorldArgs& W, float time, float* transforms, cudaStream_t stream) {
+    const uint32_t blocks = (uint32_t)(((uint64_t)W.slot_count * G + 127) / 128);
+    launch_pdl(k_world_slots<G>, dim3(blocks), dim3(128), 0, stream, W, time, transforms);
+}
+
+}  // namespace
+
+// A path's lanes evaluate its nodes again for each slot below them.  That is
+// free while the chip is not full (32,768 nodes, paths of 4: 131,072 lanes 6.7
+// us, two launches 8.5; paths of 8: 262,144 lanes 11.9 us, 11.4).  Past that a
+// lane per node pays (524,288 nodes, meshes on the leaves of paths of 4 or 8:
+// 17.3 and 26.3 us, two launches 30.2 and 31.6), for paths of two also two
+// (24.3 us, 32.1), but not four (meshes on all nodes of paths of 4: 57 us, 33).
 void launch_world_transforms(const WorldArgs& W, float time, float* transforms, cudaStream_t stream) {
+    const uint32_t group = W.max_chain <= 1 ? 1 : W.max_chain <= 2 ? 2 : W.max_chain <= 4 ? 4 : 8;
+    const uint64_t lanes = (uint64_t)W.slot_count * group;
+    if (W.max_chain <= group && lanes <= std::max<uint64_t>(131072, (uint64_t)W.node_count * (group == 2 ? 2 : 1))) {
+        if (!lanes) return;
+        if (group == 1) launch_slots<1>(W, time, transforms, stream);
+        else if (group == 2) launch_slots<2>(W, time, transforms, stream);
+        else if (group == 4) launch_slots<4>(W, time, transforms, stream);
+        else launch_slots<8>(W, time, transforms, stream);
+        return;
+    }
     if (W.node_count) launch_pdl(k_world_local, dim3((W.node_count + 127) / 128), dim3(128), 0, stream, W, time);
     if (W.slot_count)
         launch_pdl(k_world_chain, dim3((W.slot_count + 127) / 128), dim3(128), 0, stream, W, transforms);
@@ -393,6 +462,7 @@ int plan_world(const vkgv_world_desc& D, WorldPlan& P, std::string& err) {
                     const uint32_t slot = (uint32_t)(P.chain_offsets.size() - 1);
                     P.chain_nodes.insert(P.chain_nodes.end(), path.begin(), path.end());
                     P.chain_offsets.push_back((uint32_t)P.chain_nodes.size());
+                    P.max_chain = std::max(P.max_chain, (uint32_t)path.size());
                     for (uint32_t i = D.mesh_offsets[nd.mesh_index]; i < D.mesh_offsets[nd.mesh_index + 1]; ++i) {
                         const uint32_t prim = D.mesh_primitives[i];
                         const uint32_t count = D.primitive_meshlet_counts[prim];
