@@ -18,6 +18,8 @@
 // One thread per block: the palette is built once for its 16 texels.
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace vkgv {
@@ -196,8 +198,9 @@ __global__ void __launch_bounds__(32 * kDecodeRows) k_decode_bc(const uint8_t* _
 // interpolated as ((64 - w) e0 + w e1 + 32) >> 6 with the 2-, 3- and 4-bit
 // weight tables; the anchor texel of each subset stores one index bit less.
 // A reserved mode (first byte 0) decodes to transparent black.  The
-// partition and anchor tables below are the format's own.
-__constant__ uint16_t c_bc7_p2[64] = {
+// partition and anchor tables below are the format's own.  They lie in global
+// memory: a CTA copies them in a few coalesced loads.
+__device__ const uint16_t g_bc7_p2[64] = {
     0xCCCC, 0x8888, 0xEEEE, 0xECC8, 0xC880, 0xFEEC, 0xFEC8, 0xEC80, 0xC800, 0xFFEC, 0xFE80, 0xE800,
     0xFFE8, 0xFF00, 0xFFF0, 0xF000, 0xF710, 0x008E, 0x7100, 0x08CE, 0x008C, 0x7310, 0x3100, 0x8CCE,
     0x088C, 0x3110, 0x6666, 0x366C, 0x17E8, 0x0FF0, 0x718E, 0x399C, 0xAAAA, 0xF0F0, 0x5A5A, 0x33CC,
@@ -205,7 +208,7 @@ __constant__ uint16_t c_bc7_p2[64] = {
     0x0272, 0x04E4, 0x4E40, 0x2720, 0xC936, 0x936C, 0x39C6, 0x639C, 0x9336, 0x9CC6, 0x817E, 0xE718,
     0xCCF0, 0x0FCC, 0x7744, 0xEE22};
 // 3-subset partitions: two bits per texel, texel 0 in the lowest bits
-__constant__ uint32_t c_bc7_p3[64] = {
+__device__ const uint32_t g_bc7_p3[64] = {
     0xAA685050, 0x6A5A5040, 0x5A5A4200, 0x5450A0A8, 0xA5A50000, 0xA0A05050, 0x5555A0A0, 0x5A5A5050,
     0xAA550000, 0xAA555500, 0xAAAA5500, 0x90909090, 0x94949494, 0xA4A4A4A4, 0xA9A59450, 0x2A0A4250,
     0xA5945040, 0x0A425054, 0xA5A5A500, 0x55A0A0A0, 0xA8A85454, 0x6A6A4040, 0xA4A45000, 0x1A1A0500,
@@ -214,15 +217,15 @@ __constant__ uint32_t c_bc7_p3[64] = {
     0x500AA550, 0xAAAA4444, 0x66660000, 0xA5A0A5A0, 0x50A050A0, 0x69286928, 0x44AAAA44, 0x66666600,
     0xAA444444, 0x54A854A8, 0x95809580, 0x96969600, 0xA85454A8, 0x80959580, 0xAA141414, 0x96960000,
     0xAAAA1414, 0xA05050A0, 0xA0A5A5A0, 0x96000000, 0x40804080, 0xA9A8A9A8, 0xAAAAAA44, 0x2A4A5254};
-__constant__ uint8_t c_bc7_a2[64] = {
+__device__ const uint8_t g_bc7_a2[64] = {
     15, 15, 15, 15, 15, 15, 15, 15, 15, 15, 15, 15, 15, 15, 15, 15, 15, 2, 8, 2, 2, 8, 8, 15, 2, 8,
     2, 2, 8, 8, 2, 2, 15, 15, 6, 8, 2, 8, 15, 15, 2, 8, 2, 2, 2, 15, 15, 6, 6, 2, 6, 8, 15, 15, 2,
     2, 15, 15, 15, 15, 15, 2, 2, 15};
-__constant__ uint8_t c_bc7_a3a[64] = {
+__device__ const uint8_t g_bc7_a3a[64] = {
     3, 3, 15, 15, 8, 3, 15, 15, 8, 8, 6, 6, 6, 5, 3, 3, 3, 3, 8, 15, 3, 3, 6, 10, 5, 8, 8, 6, 8, 5,
     15, 15, 8, 15, 3, 5, 6, 10, 8, 15, 15, 3, 15, 5, 15, 15, 15, 15, 3, 15, 5, 5, 5, 8, 5, 10, 5,
     10, 8, 13, 15, 12, 3, 3};
-__constant__ uint8_t c_bc7_a3b[64] = {
+__device__ const uint8_t g_bc7_a3b[64] = {
     15, 8, 8, 3, 15, 15, 3, 8, 15, 15, 15, 15, 15, 15, 15, 8, 15, 8, 15, 3, 15, 8, 15, 8, 3, 15, 6,
     10, 15, 15, 10, 8, 15, 3, 15, 10, 10, 8, 9, 10, 6, 15, 8, 15, 3, 6, 6, 8, 15, 3, 15, 15, 15, 15,
     15, 15, 15, 15, 15, 15, 3, 15, 15, 8};
@@ -235,6 +238,22 @@ __device__ __forceinline__ uint32_t index_weight(uint32_t i) {
     if (BITS == 2) return i * 21u + (i >> 1);
     if (BITS == 3) return i * 9u + (i >> 2);
     return (i * 17u + 2u) >> 2;
+}
+
+// The four BITS-bit indices in the low bits of `v` as the bytes of a word, and
+// the weights of such a word, four at a time.
+template <int BITS>
+__device__ __forceinline__ uint32_t spread_indices(uint32_t v) {
+    constexpr uint32_t one = (1u << BITS) - 1u, two = (1u << (2 * BITS)) - 1u;
+    v = (v | (v << (16 - 2 * BITS))) & (two * 0x00010001u);
+    return (v | (v << (8 - BITS))) & (one * 0x01010101u);
+}
+
+template <int BITS>
+__device__ __forceinline__ uint32_t index_weights(uint32_t i) {
+    if (BITS == 2) return i * 21u + ((i >> 1) & 0x01010101u);
+    if (BITS == 3) return i * 9u + ((i >> 2) & 0x01010101u);
+    return i * 4u + (((i + 0x02020202u) >> 2) & 0x07070707u);
 }
 
 // N bits of the 128-bit block at bit POS, least significant first.
@@ -265,7 +284,10 @@ __device__ __forceinline__ uint64_t block_tail(const uint4& q) {
 
 // Gives an anchor texel the index bit that the format leaves out: a zero bit
 // at position p, the bits from p on moving up by one.
-__device__ __forceinline__ uint64_t insert_zero(uint64_t v, uint32_t p) { return v + (v & (~0ull << p)); }
+template <class T>
+__device__ __forceinline__ T insert_zero(T v, uint32_t p) {
+    return v + (v & ((T)~T(0) << p));
+}
 
 // One BC7 mode.  Stored fields in order: mode (unary), partition, rotation,
 // index selection, R of every end point (subset-major), then G, B and alpha,
@@ -321,99 +343,112 @@ __device__ __forceinline__ void bc7_end(const uint4& q, uint32_t& rb, uint32_t& 
     ga = bc7_expand<cb + p>(g) | (a << 16);
 }
 
-// The partition and anchor tables in shared memory: the lanes of a warp look
-// up different partitions, which the constant cache serialises.
+// The partition and anchor tables in shared memory, by partition: the lanes
+// of a warp look up different ones.
 struct Bc7Tables {
-    uint32_t p3[64];
-    uint16_t p2[64];
-    uint8_t a2[64], a3a[64], a3b[64];
+    uint32_t two[64];    // 2 subsets: the partition, the anchor in bits 16-19
+    uint32_t three[64];  // 3 subsets: the partition
+    uint16_t after[64];  // and its anchors in ascending order, 8 bits each
 };
 
-__device__ void bc7_load_tables(Bc7Tables& t) {
-    for (uint32_t i = threadIdx.x; i < 64; i += blockDim.x) {
-        t.p3[i] = c_bc7_p3[i];
-        t.p2[i] = c_bc7_p2[i];
-        t.a2[i] = c_bc7_a2[i];
-        t.a3a[i] = c_bc7_a3a[i];
-        t.a3b[i] = c_bc7_a3b[i];
+__device__ __forceinline__ void bc7_load_tables(Bc7Tables& t) {
+    const uint32_t i = threadIdx.x;
+    if (i < 64) {
+        t.two[i] = g_bc7_p2[i] | ((uint32_t)g_bc7_a2[i] << 16);
+        t.three[i] = g_bc7_p3[i];
+        const uint32_t a = g_bc7_a3a[i], b = g_bc7_a3b[i];
+        t.after[i] = (uint16_t)(min(a, b) | (max(a, b) << 8));
     }
 }
 
 // Decodes one block of MODE; row r goes to out[r * pitch].  Every field is at
 // a position known at compile time, and the index stream is brought to a
 // fixed width a texel by inserting the anchors' zero bits.
+// A texel's ((64 - w) e0 + w e1 + 32) >> 6 is the high byte of
+// 4 (64 e0 + 32) + w 4 (e1 - e0), at most 65,408: a word holds two channels,
+// whose sums are exact modulo 2^32, so a texel is two multiply-adds and one
+// byte permutation.
 template <int MODE>
 __device__ __forceinline__ void bc7_block(const Bc7Tables& T, const uint4& q, uint4* out, uint32_t pitch) {
     using M = Bc7Mode<MODE>;
-    uint32_t rb[6], ga[6];
-    bc7_end<MODE, 0>(q, rb[0], ga[0]);
-    bc7_end<MODE, 1>(q, rb[1], ga[1]);
+    constexpr int ib = M::kIndex, ib2 = M::kIndex2;
+    uint32_t base[2 * M::kSubsets], step[2 * M::kSubsets];  // red and blue, green and alpha of each subset
+    uint32_t e0, e1, f0, f1;
+    const auto line = [&](int k) {
+        base[2 * k] = 256u * e0 + 0x00800080u, step[2 * k] = 4u * (e1 - e0);
+        base[2 * k + 1] = 256u * f0 + 0x00800080u, step[2 * k + 1] = 4u * (f1 - f0);
+    };
+    bc7_end<MODE, 0>(q, e0, f0);
+    bc7_end<MODE, 1>(q, e1, f1);
+    uint32_t base_a = 0, step_a = 0;
+    if constexpr (ib2 != 0) {  // alpha has weights of its own
+        base_a = 256u * (f0 >> 16) + 0x80u, step_a = 4u * ((f1 >> 16) - (f0 >> 16));
+        f0 &= 255u, f1 &= 255u;
+    }
+    line(0);
     if constexpr (M::kSubsets > 1) {
-        bc7_end<MODE, 2>(q, rb[2], ga[2]);
-        bc7_end<MODE, 3>(q, rb[3], ga[3]);
+        bc7_end<MODE, 2>(q, e0, f0);
+        bc7_end<MODE, 3>(q, e1, f1);
+        line(1);
     }
     if constexpr (M::kSubsets > 2) {
-        bc7_end<MODE, 4>(q, rb[4], ga[4]);
-        bc7_end<MODE, 5>(q, rb[5], ga[5]);
+        bc7_end<MODE, 4>(q, e0, f0);
+        bc7_end<MODE, 5>(q, e1, f1);
+        line(2);
     }
-    constexpr int ib = M::kIndex, ib2 = M::kIndex2;
     const uint32_t part = block_bits<M::kPartAt, M::kPartBits>(q);
-    uint64_t ix = block_tail<M::kIndexAt>(q), ix2 = 0;
+    using Stream = std::conditional_t<ib == 2, uint32_t, uint64_t>;
+    using Stream2 = std::conditional_t<ib2 == 2, uint32_t, uint64_t>;
+    Stream ix = (Stream)block_tail<M::kIndexAt>(q);
+    Stream2 ix2 = 0;
     if constexpr (ib2 != 0) {
-        ix &= (1ull << (16 * ib - 1)) - 1ull;
-        ix2 = insert_zero(block_tail<M::kIndex2At>(q), ib2 - 1);
+        ix &= (Stream)((1ull << (16 * ib - 1)) - 1ull);
+        ix2 = insert_zero((Stream2)block_tail<M::kIndex2At>(q), ib2 - 1);
     }
     ix = insert_zero(ix, ib - 1);
     uint32_t pmask = 0u;
     if constexpr (M::kSubsets == 2) {
-        pmask = T.p2[part];
-        ix = insert_zero(ix, T.a2[part] * ib + ib - 1);
+        pmask = T.two[part];
+        ix = insert_zero(ix, (pmask >> 16) * ib + ib - 1);
     } else if constexpr (M::kSubsets == 3) {
-        pmask = T.p3[part];
-        const uint32_t a = T.a3a[part], b = T.a3b[part];
-        ix = insert_zero(ix, min(a, b) * ib + ib - 1);
-        ix = insert_zero(ix, max(a, b) * ib + ib - 1);
+        pmask = T.three[part];
+        const uint32_t after = T.after[part];
+        ix = insert_zero(ix, (after & 255u) * ib + ib - 1);
+        ix = insert_zero(ix, (after >> 8) * ib + ib - 1);
     }
-    // alpha swaps with R (1), G (2) or B (3)
-    uint32_t order = 0x3210u;
+    // alpha (byte 5 of the last permutation) swaps with R (1), G (2) or B (3)
+    uint32_t order = 0x5210u;
     bool second = false;  // mode 4: the colours take the second index set
     if constexpr (M::kRotBits != 0) {
         const uint32_t rot = block_bits<M::kRotAt, 2>(q);
-        order = rot == 0 ? 0x3210u : (rot == 1 ? 0x0213u : (rot == 2 ? 0x1230u : 0x2310u));
+        order = rot == 0 ? 0x5210u : (rot == 1 ? 0x0215u : (rot == 2 ? 0x1250u : 0x2510u));
         second = block_bits<M::kSelAt, M::kSelBits>(q) != 0;
     }
-#pragma unroll
+#pragma unroll 1
     for (int r = 0; r < 4; ++r) {
         uint32_t t[4];
+        uint32_t wc = index_weights<ib>(spread_indices<ib>((uint32_t)(ix >> (4 * ib * r)) & ((1u << (4 * ib)) - 1u)));
+        uint32_t wa = 0;
+        if constexpr (ib2 != 0) {
+            wa = index_weights<ib2>(spread_indices<ib2>((uint32_t)(ix2 >> (4 * ib2 * r)) & ((1u << (4 * ib2)) - 1u)));
+            const uint32_t w = wc;
+            wc = second ? wa : w, wa = second ? w : wa;
+        }
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
             const int i = 4 * r + x;
-            uint32_t e0 = rb[0], e1 = rb[1], f0 = ga[0], f1 = ga[1];
+            uint32_t b0 = base[0], d0 = step[0], b1 = base[1], d1 = step[1];
             if constexpr (M::kSubsets == 2) {
                 const bool s = (pmask >> i) & 1u;
-                e0 = s ? rb[2] : e0, e1 = s ? rb[3] : e1, f0 = s ? ga[2] : f0, f1 = s ? ga[3] : f1;
+                b0 = s ? base[2] : b0, d0 = s ? step[2] : d0, b1 = s ? base[3] : b1, d1 = s ? step[3] : d1;
             } else if constexpr (M::kSubsets == 3) {
                 const bool s = (pmask >> (2 * i)) & 1u, s2 = (pmask >> (2 * i)) & 2u;
-                e0 = s ? rb[2] : (s2 ? rb[4] : e0), e1 = s ? rb[3] : (s2 ? rb[5] : e1);
-                f0 = s ? ga[2] : (s2 ? ga[4] : f0), f1 = s ? ga[3] : (s2 ? ga[5] : f1);
+                b0 = s ? base[2] : (s2 ? base[4] : b0), d0 = s ? step[2] : (s2 ? step[4] : d0);
+                b1 = s ? base[3] : (s2 ? base[5] : b1), d1 = s ? step[3] : (s2 ? step[5] : d1);
             }
-            uint32_t wc = index_weight<ib>((uint32_t)(ix >> (ib * i)) & ((1u << ib) - 1u)), v, u;
-            // ((64 - w) e0 + w e1 + 32) >> 6 in each half: at most 64 * 255 + 32
-            if constexpr (ib2 != 0) {
-                uint32_t wa = index_weight<ib2>((uint32_t)(ix2 >> (ib2 * i)) & ((1u << ib2) - 1u));
-                if (second) {
-                    const uint32_t w = wc;
-                    wc = wa, wa = w;
-                }
-                const uint32_t g = (64u - wc) * (f0 & 255u) + wc * (f1 & 255u);
-                const uint32_t a = (64u - wa) * (f0 >> 16) + wa * (f1 >> 16);
-                u = (g | (a << 16)) + 0x00200020u;
-            } else {
-                u = (64u - wc) * f0 + wc * f1 + 0x00200020u;
-            }
-            v = (64u - wc) * e0 + wc * e1 + 0x00200020u;
-            t[x] = ((v >> 6) & 0x00FF00FFu) | ((u << 2) & 0xFF00FF00u);
-            if constexpr (M::kRotBits != 0) t[x] = __byte_perm(t[x], 0u, order);
+            const uint32_t w = (wc >> (8 * x)) & 255u, v = b0 + w * d0, u = b1 + w * d1;
+            t[x] = __byte_perm(v, u, 0x7351u);
+            if constexpr (ib2 != 0) t[x] = __byte_perm(t[x], base_a + ((wa >> (8 * x)) & 255u) * step_a, order);
         }
         out[r * pitch] = make_uint4(t[0], t[1], t[2], t[3]);
     }
@@ -422,19 +457,25 @@ __device__ __forceinline__ void bc7_block(const Bc7Tables& T, const uint4& q, ui
 // BC7: a CTA decodes a tile of 512 blocks (tw wide, a power of two) sorted by
 // mode, so that each warp runs one mode's code, whose fields are at constant
 // positions; a thread decodes a whole block, and the rows leave through
-// shared memory as contiguous stores.  The lists of the eight modes are
-// padded to whole warps (some 20 warp jobs a tile instead of 16).  Bound by
-// instruction issue (8192^2, modes as encoders choose them: 556 -> 195 us; with
-// four lanes per block in image order every field was extracted at a position
-// looked up at run time, four times).
-constexpr uint32_t kBc7Blocks = 512, kBc7Threads = 256;
+// shared memory, each as one bulk copy where the image's rows are 16-byte
+// aligned.  The lists of the modes are padded to whole warps (some 20 warp
+// jobs a tile instead of 16).  Bound by instruction issue (ALU pipe 65% of its
+// cycles).  8192^2, modes as encoders choose them: 551 us with four lanes per
+// block in image order, every field at a position looked up at run time;
+// 191 sorted; 84 with packed weights, a multiply-add for two channels, jobs
+// found by a ballot, the row loop rolled (the eight modes unrolled overran the
+// instruction cache: 112) and the bulk copies (97 without).  Stores straight
+// to the image saved the last barrier (4096^2: 1,024-block tiles 23.6 us, this
+// 25.0), but their half sectors went to memory and back once the image was
+// past L2 (8192^2: 148 us).
+constexpr uint32_t kBc7Blocks = 512, kBc7Threads = 256, kBc7Each = kBc7Blocks / kBc7Threads;
 
-__global__ void __launch_bounds__(kBc7Threads) k_decode_bc7(const uint8_t* __restrict__ blocks, uint32_t w, uint32_t h,
-                                                            uint32_t tw_log2, uint32_t* __restrict__ rgba) {
+__global__ void __launch_bounds__(kBc7Threads, 6)
+    k_decode_bc7(const uint8_t* __restrict__ blocks, uint32_t w, uint32_t h, uint32_t tw_log2,
+                 uint32_t* __restrict__ rgba) {
     __shared__ Bc7Tables T;
     __shared__ uint32_t s_count[9];                     // blocks of each mode (8: reserved)
     __shared__ uint16_t s_list[kBc7Blocks + 9 * 32];    // tile positions by mode, each mode's padded to a warp
-    __shared__ __align__(16) uint4 s_block[kBc7Blocks];
     __shared__ __align__(16) uint4 s_out[4 * kBc7Blocks];
     bc7_load_tables(T);
     if (threadIdx.x < 9) s_count[threadIdx.x] = 0;
@@ -444,19 +485,20 @@ __global__ void __launch_bounds__(kBc7Threads) k_decode_bc7(const uint8_t* __res
     const uint32_t tw = 1u << tw_log2, th = kBc7Blocks >> tw_log2;
     const uint32_t bw = (w + 3) / 4, bh = (h + 3) / 4;
     const uint32_t bx0 = blockIdx.x * tw, by0 = blockIdx.y * th;
-    uint32_t mode[2], rank[2];
+    const uint4* src = reinterpret_cast<const uint4*>(blocks) + ((size_t)by0 * bw + bx0);
+    uint32_t mode[kBc7Each], rank[kBc7Each];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const uint32_t i = threadIdx.x + k * kBc7Threads, bx = bx0 + (i & (tw - 1)), by = by0 + (i >> tw_log2);
-        const bool live = bx < bw && by < bh;
-        uint4 q = make_uint4(0, 0, 0, 0);
-        if (live) q = __ldg(reinterpret_cast<const uint4*>(blocks) + ((size_t)by * bw + bx));
-        s_block[i] = q;
+    for (uint32_t k = 0; k < kBc7Each; ++k) {
+        const uint32_t i = threadIdx.x + k * kBc7Threads, x = i & (tw - 1), y = i >> tw_log2;
         // the mode is the lowest set bit of the first byte; none: reserved
-        mode[k] = !live ? 9u : ((q.x & 0xFFu) ? (uint32_t)__ffs((int)(q.x & 0xFFu)) - 1u : 8u);
+        mode[k] = 9u;
+        if (bx0 + x < bw && by0 + y < bh) {
+            const uint32_t q = __ldg(&src[(size_t)y * bw + x].x) & 0xFFu;
+            mode[k] = q ? (uint32_t)__ffs((int)q) - 1u : 8u;
+        }
     }
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
+    for (uint32_t k = 0; k < kBc7Each; ++k) {
         const unsigned same = __match_any_sync(0xffffffffu, mode[k]);
         const int leader = __ffs((int)same) - 1;
         uint32_t base = 0;
@@ -464,56 +506,58 @@ __global__ void __launch_bounds__(kBc7Threads) k_decode_bc7(const uint8_t* __res
         rank[k] = __shfl_sync(0xffffffffu, base, leader) + (uint32_t)__popc(same & ((1u << lane) - 1u));
     }
     __syncthreads();
-    // warp jobs: mode m owns jobs [first_m, first_m + ceil(count_m / 32))
-    uint32_t jobs = 0;
-    uint32_t first[9];
+    // warp jobs: mode m owns jobs [first_m, first_m + ceil(count_m / 32)),
+    // lane m of every warp holds its count and first
+    const uint32_t count = lane < 9 ? s_count[lane] : 0u;
+    uint32_t jobs = (count + 31) / 32;
 #pragma unroll
-    for (int m = 0; m < 9; ++m) {
-        first[m] = jobs;
-        jobs += (s_count[m] + 31) / 32;
+    for (int d = 1; d < 16; d <<= 1) {
+        const uint32_t below = __shfl_up_sync(0xffffffffu, jobs, d);
+        if ((int)lane >= d) jobs += below;
     }
+    const uint32_t first = jobs - (count + 31) / 32;
+    jobs = __shfl_sync(0xffffffffu, jobs, 9);
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-        for (int m = 0; m < 9; ++m)
-            if (mode[k] == (uint32_t)m) s_list[32 * first[m] + rank[k]] = (uint16_t)(threadIdx.x + k * kBc7Threads);
+    for (uint32_t k = 0; k < kBc7Each; ++k) {
+        const uint32_t base = __shfl_sync(0xffffffffu, first, (int)mode[k]);
+        if (mode[k] < 9) s_list[32 * base + rank[k]] = (uint16_t)(threadIdx.x + k * kBc7Threads);
+    }
     __syncthreads();
     for (uint32_t j = warp; j < jobs; j += kBc7Threads / 32) {
-        uint32_t m = 0, at = 0;
-#pragma unroll
-        for (int k = 1; k < 9; ++k)
-            if (j >= first[k] && s_count[k]) m = (uint32_t)k;
-#pragma unroll
-        for (int k = 0; k < 9; ++k)
-            if (m == (uint32_t)k) at = 32 * (j - first[k]);
-        if (at + lane >= s_count[m]) continue;
-        const uint32_t i = s_list[32 * j + lane];
-        const uint4 q = s_block[i];
-        uint4* out = s_out + ((i >> tw_log2) << (tw_log2 + 2)) + (i & (tw - 1));
-        switch (m) {  // the same for the whole warp
-            case 0: bc7_block<0>(T, q, out, tw); break;
-            case 1: bc7_block<1>(T, q, out, tw); break;
-            case 2: bc7_block<2>(T, q, out, tw); break;
-            case 3: bc7_block<3>(T, q, out, tw); break;
-            case 4: bc7_block<4>(T, q, out, tw); break;
-            case 5: bc7_block<5>(T, q, out, tw); break;
-            case 6: bc7_block<6>(T, q, out, tw); break;
-            case 7: bc7_block<7>(T, q, out, tw); break;
-            default:  // a reserved mode decodes to transparent black
-                for (int r = 0; r < 4; ++r) out[r * tw] = make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t m = 31u - (uint32_t)__clz((int)__ballot_sync(0xffffffffu, count != 0 && first <= j));
+        const uint32_t at = 32 * (j - __shfl_sync(0xffffffffu, first, (int)m));
+        if (at + lane < __shfl_sync(0xffffffffu, count, (int)m)) {
+            const uint32_t i = s_list[32 * j + lane], x = i & (tw - 1), y = i >> tw_log2;
+            const uint4 q = __ldg(src + (size_t)y * bw + x);
+            uint4* out = s_out + ((y << (tw_log2 + 2)) + x);
+            switch (m) {  // the same for the whole warp
+                case 0: bc7_block<0>(T, q, out, tw); break;
+                case 1: bc7_block<1>(T, q, out, tw); break;
+                case 2: bc7_block<2>(T, q, out, tw); break;
+                case 3: bc7_block<3>(T, q, out, tw); break;
+                case 4: bc7_block<4>(T, q, out, tw); break;
+                case 5: bc7_block<5>(T, q, out, tw); break;
+                case 6: bc7_block<6>(T, q, out, tw); break;
+                case 7: bc7_block<7>(T, q, out, tw); break;
+                default:  // a reserved mode decodes to transparent black
+                    for (uint32_t r = 0; r < 4; ++r) out[r * tw] = make_uint4(0u, 0u, 0u, 0u);
+            }
         }
     }
-    __syncthreads();
     // the tile's texel rows, each 4 tw texels, contiguous in the image
     const uint32_t px = min(4 * tw, w - 4 * bx0), rows = min(4 * th, h - 4 * by0);
     uint32_t* dst = rgba + (size_t)by0 * 4 * w + (size_t)bx0 * 4;
-    const bool wide = (w & 3u) == 0 && ((uint32_t)reinterpret_cast<uintptr_t>(dst) & 15u) == 0;
-    if (wide) {
-        for (uint32_t i = threadIdx.x; i < 4 * kBc7Blocks; i += kBc7Threads) {
-            const uint32_t x = i & (tw - 1), y = i >> tw_log2;
-            if (4 * x < px && y < rows) __stcs(reinterpret_cast<uint4*>(dst + (size_t)y * w) + x, s_out[i]);
+    if ((w & 3u) == 0 && ((uint32_t)reinterpret_cast<uintptr_t>(rgba) & 15u) == 0) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (threadIdx.x < rows) {  // a bulk copy a row
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst + (size_t)threadIdx.x * w),
+                         "r"((uint32_t)__cvta_generic_to_shared(s_out + (threadIdx.x << tw_log2))), "r"(4 * px)
+                         : "memory");
+            asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
         }
     } else {
+        __syncthreads();
         const uint32_t* texels = reinterpret_cast<const uint32_t*>(s_out);
         for (uint32_t i = threadIdx.x; i < 16 * kBc7Blocks; i += kBc7Threads) {
             const uint32_t x = i & (4 * tw - 1), y = i >> (tw_log2 + 2);
@@ -689,8 +733,8 @@ __global__ void __launch_bounds__(32 * kDecodeRows) k_decode_bc6h(const uint8_t*
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     if (tid < 15) s_count[tid] = 0;
     if (tid < 32) {
-        s_p2[tid] = c_bc7_p2[tid];
-        s_a2[tid] = c_bc7_a2[tid];
+        s_p2[tid] = g_bc7_p2[tid];
+        s_a2[tid] = g_bc7_a2[tid];
     }
     pdl_begin();
     __syncthreads();
@@ -898,7 +942,8 @@ void launch_decode_bc(const uint8_t* blocks, uint32_t format, uint32_t w, uint32
     const uint32_t bw = (w + 3) / 4, bh = (h + 3) / 4;
     if (format == VKGV_BC7) {
         // tiles 128 blocks wide, narrower ones for narrower images
-        const uint32_t tw_log2 = bw <= 32 ? 5u : (bw <= 64 ? 6u : 7u), th = kBc7Blocks >> tw_log2;
+        const uint32_t tw_log2 = bw <= 32 ? 5u : (bw <= 64 ? 6u : 7u);
+        const uint32_t th = kBc7Blocks >> tw_log2;
         const dim3 grid((bw + (1u << tw_log2) - 1) >> tw_log2, (bh + th - 1) / th);
         launch_pdl(k_decode_bc7, grid, dim3(kBc7Threads), 0, stream, blocks, w, h, tw_log2, rgba);
         return;
