@@ -72,16 +72,55 @@ __global__ void k_diff_setup(DiffSetup S) {
     }
 }
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+// Element min(i, 2) of v.
+template <class T>
+__device__ __forceinline__ T pick(uint32_t i, const T v[3]) {
+    return i == 0 ? v[0] : (i == 1 ? v[1] : v[2]);
 }
 
-__device__ __forceinline__ double warp_min(double v) {
+// The sums over a warp of three values: after one exchange the rest of the
+// tree runs for all three at once, in eight lanes each (7 additions instead
+// of 15, each the same one).
+__device__ __forceinline__ void warp_sum3(uint32_t lane, double v[3]) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+    for (int c = 0; c < 3; ++c) v[c] += __shfl_xor_sync(0xffffffffu, v[c], 16);
+    double w[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) w[c] = __shfl_xor_sync(0xffffffffu, v[c], 8);
+    double s = pick(lane >> 3, v) + pick(lane >> 3, w);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v[c] = __shfl_sync(0xffffffffu, s, 8 * c);
+}
+
+// (double)f by integer operations: a conversion takes a turn in the double
+// pipe, which here does two lanes a cycle.
+__device__ __forceinline__ double widen(float f) {
+    const uint32_t b = __float_as_uint(f), mag = b & 0x7FFFFFFFu;
+    double d = __hiloint2double((int)((b & 0x80000000u) | (mag ? (mag >> 3) + 0x38000000u : 0u)), (int)(b << 29));
+    if (mag - 1u < 0x007FFFFFu || mag >= 0x7F800000u) d = (double)f;  // subnormal, infinite, NaN
+    return d;
+}
+
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// The least double of a warp by its bits.  Positive values order as their
+// bits do; a negative one, of which it may not find the least, stays below
+// all positive ones.
+__device__ __forceinline__ double warp_min_bits(double v) {
+    long long k = __double_as_longlong(v);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) k = min(k, __shfl_xor_sync(0xffffffffu, k, o));
+    return __longlong_as_double(k);
+}
+
+__device__ __forceinline__ double min_bits(double a, double b) {
+    return __longlong_as_double(min(__double_as_longlong(a), __double_as_longlong(b)));
 }
 
 // Unit normal of triangle t of a meshlet in double; false when degenerate.
@@ -93,14 +132,17 @@ __device__ __forceinline__ bool tri_normal(const DiffSetup& S, const uint32_t* v
     double e1[3], e2[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        e1[k] = (double)b[k] - (double)a[k];
-        e2[k] = (double)c[k] - (double)a[k];
+        const double o = widen(a[k]);
+        e1[k] = widen(b[k]) - o;
+        e2[k] = widen(c[k]) - o;
     }
     n[0] = e1[1] * e2[2] - e1[2] * e2[1];
     n[1] = e1[2] * e2[0] - e1[0] * e2[2];
     n[2] = e1[0] * e2[1] - e1[1] * e2[0];
     const double len2 = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
-    if (!(len2 > 1e-60)) return false;
+    // !(len2 > 1e-60), by the bits
+    const long long bits = __double_as_longlong(len2);
+    if (bits <= __double_as_longlong(1e-60) || bits > 0x7FF0000000000000ll) return false;
     const double r = rsqrt(len2);
     n[0] *= r, n[1] *= r, n[2] *= r;
     return true;
@@ -121,40 +163,52 @@ __global__ void k_diff_cones(DiffSetup S) {
         const uint32_t tc = min((uint32_t)ml.triangle_count, (uint32_t)VKGV_MAX_PRIMITIVES);
         const uint32_t* vidx = S.vertex_indices + ml.vertex_offset;
         const uint8_t* tri = S.tri_indices + ml.triangle_offset;
-        double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+        // the bounds in float: a minimum of floats is one of them
+        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
         for (uint32_t k = lane; k < vc; k += 32) {
             const float* p = S.positions + 3 * (size_t)vidx[k];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) lo[c] = fmin(lo[c], (double)p[c]), hi[c] = fmax(hi[c], (double)p[c]);
+            for (int c = 0; c < 3; ++c) lo[c] = fminf(lo[c], p[c]), hi[c] = fmaxf(hi[c], p[c]);
         }
-        float center[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             lo[c] = warp_min(lo[c]);
             hi[c] = -warp_min(-hi[c]);
-            center[c] = (float)(0.5 * (lo[c] + hi[c]));
         }
-        double r2 = 0.0;
+        // lane c does axis c's arithmetic
+        const float mid = (float)(0.5 * (widen(pick(lane, lo)) + widen(pick(lane, hi))));
+        float center[3];
+        double centre[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            center[c] = __shfl_sync(0xffffffffu, mid, c);
+            centre[c] = widen(center[c]);
+        }
+        long long r2_bits = 0;  // of the greatest squared distance, a NaN apart
         for (uint32_t k = lane; k < vc; k += 32) {
             const float* p = S.positions + 3 * (size_t)vidx[k];
             double d2 = 0.0;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const double e = (double)p[c] - (double)center[c];
+                const double e = widen(p[c]) - centre[c];
                 d2 += e * e;
             }
-            r2 = fmax(r2, d2);
+            const long long bits = __double_as_longlong(d2);
+            if (bits <= 0x7FF0000000000000ll) r2_bits = max(r2_bits, bits);
         }
-        r2 = -warp_min(-r2);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) r2_bits = max(r2_bits, __shfl_xor_sync(0xffffffffu, r2_bits, o));
+        const double r2 = __longlong_as_double(r2_bits);
         vkgv_meshlet_cone cone;
         cone.center[0] = center[0], cone.center[1] = center[1], cone.center[2] = center[2];
-        cone.radius = nextafterf((float)(sqrt(r2) * (1.0 + 1e-6) + 1e-7), INFINITY);
         cone.axis[0] = cone.axis[1] = cone.axis[2] = 0.0f;
         cone.cutoff = -1.0f;
         // a lane's normals (at most four) stay in registers for the second
-        // pass: double arithmetic is what this kernel waits for (14,100
-        // meshlets: 675 -> 380 us, with one rsqrt in place of a square root and
-        // three quotients)
+        // pass: double arithmetic is what this kernel waits for.  18,400
+        // meshlets: 675 us; 389 with that and one rsqrt in place of a square
+        // root and three quotients; 220 without its conversions and
+        // comparisons, scalar steps of several values in one instruction, and
+        // one dot product a normal.
         constexpr int kPerLane = (VKGV_MAX_PRIMITIVES + 31) / 32;
         double n[kPerLane][3];
         double sum[3] = {0.0, 0.0, 0.0};
@@ -170,26 +224,32 @@ __global__ void k_diff_cones(DiffSetup S) {
             }
         }
         degenerate = __any_sync(0xffffffffu, degenerate);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) sum[c] = warp_sum(sum[c]);
-        const double sl = sqrt(sum[0] * sum[0] + sum[1] * sum[1] + sum[2] * sum[2]);
+        warp_sum3(lane, sum);
+        // lane 0 takes the root of the radius, the others that of the length
+        const double len2 = sum[0] * sum[0] + sum[1] * sum[1] + sum[2] * sum[2];
+        const double root = sqrt(lane == 0 ? r2 : len2);
+        const double sl = __shfl_sync(0xffffffffu, root, 1);
+        cone.radius = nextafterf((float)(root * (1.0 + 1e-6) + 1e-7), INFINITY);  // lane 0's
         if (!degenerate && sl > 1e-12) {
-            const double axis[3] = {sum[0] / sl, sum[1] / sl, sum[2] / sl};
-            const float fa[3] = {(float)axis[0], (float)axis[1], (float)axis[2]};
-            const double fal = sqrt((double)fa[0] * fa[0] + (double)fa[1] * fa[1] + (double)fa[2] * fa[2]);
+            const double mean = pick(lane, sum) / sl;
+            const float mean_f = (float)mean;
+            const float fa[3] = {__shfl_sync(0xffffffffu, mean_f, 0), __shfl_sync(0xffffffffu, mean_f, 1),
+                                 __shfl_sync(0xffffffffu, mean_f, 2)};
+            const double da[3] = {widen(fa[0]), widen(fa[1]), widen(fa[2])};
+            const double fal = sqrt(da[0] * da[0] + da[1] * da[1] + da[2] * da[2]);
             const double inv = 1.0 / fal;
-            double cmin = 1.0, cmin_f = 1.0;
+            // The least cosine against the rounded axis; times inv last, as
+            // the product's rounding keeps the order.  It is within 2e-7 of
+            // the least against the double axis, so 1e-6 covers both.
+            double cmin = INFINITY;
 #pragma unroll
-            for (int k = 0; k < kPerLane; ++k) {
-                if (lane + 32u * (uint32_t)k >= tc) continue;
-                cmin = fmin(cmin, n[k][0] * axis[0] + n[k][1] * axis[1] + n[k][2] * axis[2]);
-                cmin_f = fmin(cmin_f, (n[k][0] * fa[0] + n[k][1] * fa[1] + n[k][2] * fa[2]) * inv);
-            }
-            cmin = warp_min(cmin);
-            cmin_f = warp_min(cmin_f) - 1e-6;
-            if (cmin > 0.05 && cmin_f > 0.05) {
+            for (int k = 0; k < kPerLane; ++k)
+                if (lane + 32u * (uint32_t)k < tc)
+                    cmin = min_bits(cmin, n[k][0] * da[0] + n[k][1] * da[1] + n[k][2] * da[2]);
+            cmin = min_bits(warp_min_bits(cmin) * inv, 1.0) - 1e-6;
+            if (cmin > 0.05) {
                 cone.axis[0] = fa[0], cone.axis[1] = fa[1], cone.axis[2] = fa[2];
-                cone.cutoff = nextafterf((float)cmin_f, -INFINITY);
+                cone.cutoff = nextafterf((float)cmin, -INFINITY);
             }
         }
         if (lane == 0) S.cones[m] = cone;
