@@ -321,14 +321,17 @@ template <bool BACKWARD>
 __device__ __forceinline__ void shade_pixel(const DiffArgs& A, const DeviceView& V, const float* VP, float sn, float cs,
                                             uint32_t p, float& loss_acc) {
     const uint32_t w = V.w;
-    const uint32_t lo = (uint32_t)V.depth_id[p];
+    // Ids, targets and colours pass through once, first out of L2: the vertices,
+    // the texture and the accumulators stay (64 views of 512^2: 581.5 -> 563 us;
+    // 128 views of 1.3M triangles 2,743 -> 2,696).
+    const uint32_t lo = __ldcs(reinterpret_cast<const uint32_t*>(V.depth_id + p));
     float tgt[3] = {0.0f, 0.0f, 0.0f};
     const bool mse = V.diff_target != nullptr;
     float* out = (!BACKWARD || A.write_rgb) ? V.diff_rgb : nullptr;
     if (BACKWARD && mse) {
-        tgt[0] = V.diff_target[3 * p];
-        tgt[1] = V.diff_target[3 * p + 1];
-        tgt[2] = V.diff_target[3 * p + 2];
+        tgt[0] = __ldcs(V.diff_target + 3 * p);
+        tgt[1] = __ldcs(V.diff_target + 3 * p + 1);
+        tgt[2] = __ldcs(V.diff_target + 3 * p + 2);
     }
     if (lo == 0) {
         if (BACKWARD) loss_acc += A.scale * (tgt[0] * tgt[0] + tgt[1] * tgt[1] + tgt[2] * tgt[2]);
@@ -403,9 +406,9 @@ __device__ __forceinline__ void shade_pixel(const DiffArgs& A, const DeviceView&
         rgb[j] = fmul(fmul(col[j], A.albedo[j]), tex[j]);
     }
     if (out) {
-        out[3 * p] = rgb[0];
-        out[3 * p + 1] = rgb[1];
-        out[3 * p + 2] = rgb[2];
+        __stcs(out + 3 * p, rgb[0]);
+        __stcs(out + 3 * p + 1, rgb[1]);
+        __stcs(out + 3 * p + 2, rgb[2]);
     }
     if (!BACKWARD) return;
     // ---- backward
