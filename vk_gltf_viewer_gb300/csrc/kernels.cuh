@@ -55,8 +55,8 @@ void launch_cull(const SceneArgs& S, const DeviceView* views, uint32_t nviews, u
                  uint32_t* status, uint32_t sm_count, cudaStream_t stream);
 // Entries a view's deferred list (DeviceView::deferred) must hold.
 uint32_t deferred_capacity(uint32_t draw_count, uint32_t sm_count);
-// work: two counters that are zero between launches (each launch returns
-// them to zero).
+// work: two counters, zero before the first launch; each instance of the
+// kernel returns the other's to zero.
 void launch_raster(const SceneArgs& S, const DeviceView* views, uint32_t nviews, const RasterLists& lists,
                    const RasterConfig& cfg, BigTri* big, uint32_t* big_count, uint32_t big_capacity,
                    uint32_t* work, uint32_t* status, uint32_t sm_count, cudaStream_t stream,
