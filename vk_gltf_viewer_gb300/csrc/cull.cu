@@ -182,6 +182,12 @@ __device__ __forceinline__ CullResult cull_one(const SceneArgs& S, const DeviceV
         M[c * 4 + 2] = q.z;
         M[c * 4 + 3] = q.w;
     }
+    // the cone array is asked for with the meshlet's bounds, not after them
+    uint64_t cones = 0;
+    if (!retest && eye && S.cone_table && dr.primitive_index < S.primitive_count) {
+        cones = S.cone_table[dr.primitive_index];
+        if (S.mats[prim->material_index].double_sided) cones = 0;
+    }
     const float e0 = ml->aabb_extents[0], e1 = ml->aabb_extents[1], e2 = ml->aabb_extents[2];
     float wc4[4];
     // worldAabbCenter (visbuffer.task.glsl:50)
@@ -209,20 +215,16 @@ __device__ __forceinline__ CullResult cull_one(const SceneArgs& S, const DeviceV
     // Meshlet normal-cone backface test (an addition; conservative with
     // respect to the per-triangle test of visbuffer.mesh.glsl:86-101, which
     // a double-sided material skips).
-    if (!retest && eye && S.cone_table && dr.primitive_index < S.primitive_count &&
-        !S.mats[prim->material_index].double_sided) {
-        const uint64_t cones = S.cone_table[dr.primitive_index];
-        if (cones) {
-            const vkgv_meshlet_cone cone = load_cone(cones, dr.meshlet_index);
-            bool culled;
-            if (V.eyes && dr.transform_index < S.transform_count) {
-                const float4 o = __ldg(V.eyes + dr.transform_index);
-                culled = o.w != 0.0f && cone_culled_at(cone, o.x, o.y, o.z);
-            } else {
-                culled = cone_culled(cone, M, eye);
-            }
-            if (culled) return res;
+    if (cones) {
+        const vkgv_meshlet_cone cone = load_cone(cones, dr.meshlet_index);
+        bool culled;
+        if (V.eyes && dr.transform_index < S.transform_count) {
+            const float4 o = __ldg(V.eyes + dr.transform_index);
+            culled = o.w != 0.0f && cone_culled_at(cone, o.x, o.y, o.z);
+        } else {
+            culled = cone_culled(cone, M, eye);
         }
+        if (culled) return res;
     }
     if (!pyr) {
         res.visible = true;
