@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
         Q.status = P.status;
     }
     __syncthreads();
-    if (warp == 0) {
+    if (nv > 1 && warp == 0) {  // (one view: 720p sphere 30.9 -> 29.7 us without)
         // inclusive scan of s_pre[1..nv]: lane-contiguous segments, then a
         // warp scan of the segment sums
         const uint32_t seg = (nv + 31) / 32, b = 1 + lane * seg, e = min(b + seg, nv + 1);
@@ -784,7 +784,7 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
             s_pre[i] = run;
         }
     }
-    __syncthreads();
+    if (nv > 1) __syncthreads();
     // The last `split` meshlets of the list are drawn by kParts warps each, one
     // 32-triangle round a warp: a launch of few meshlets then fills the chip
     // (and the longest of them takes one round, not four), and at the end of
