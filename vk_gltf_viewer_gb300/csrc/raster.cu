@@ -441,6 +441,16 @@ constexpr uint32_t kLaneArea = VKGV_RASTER_LANE_AREA;
 #endif
 constexpr uint32_t kQueueArea = VKGV_RASTER_QUEUE_AREA;
 
+// Whether the fast instance draws a triangle whose clamped bbox is bw x bh
+// pixels (and whose extent is below kSmallExtent): itself, or as one rectangle
+// of the queue.  The slow instance queues what takes several: with the line at
+// small_area it transformed every meshlet of 8-to-32-pixel triangles again
+// (a 256^2 sphere's frame 34.9 -> 30.8 us, the 1365x767 torus grid 206.9 ->
+// 197.0, 1080p 259.0 -> 253.8, 64 views of 512^2 568.6 -> 561.0).
+__device__ __forceinline__ bool fast_size(uint32_t bw, uint32_t bh, const RasterQueue& Q) {
+    return bw * bh <= Q.small_area || max(bw, bh) <= Q.chunk;
+}
+
 struct TriClass {
     int2 q0, q1, q2;  // snapped vertices
     int2 f0, f1, f2;  // {depth bits, flags}
@@ -450,8 +460,8 @@ struct TriClass {
 // backface test (visbuffer.mesh.glsl:86-101) and the empty-bbox test are
 // both pure filters, so the cheap bbox test runs first for triangles that
 // need no clipping.  kFast: snapped, inside the guard band, front-facing,
-// non-zero area, a pixel centre in its bbox, bbox within small_area pixels
-// and edge values within int32.
+// non-zero area, a pixel centre in its bbox, bbox of a fast_size and edge
+// values within int32.
 template <bool SLOW>
 __device__ __forceinline__ int classify(uint32_t i0, uint32_t i1, uint32_t i2, uint32_t vc, const int2* sxy,
                                         const int2* szf, const float4* clip, bool double_sided, float tdet, const RasterCtx& c,
@@ -482,7 +492,7 @@ __device__ __forceinline__ int classify(uint32_t i0, uint32_t i1, uint32_t i2, u
     const int64_t A = (int64_t)(q1.x - q0.x) * (q2.y - q0.y) - (int64_t)(q1.y - q0.y) * (q2.x - q0.x);
     if (A == 0) return kDrop;
     const bool small = maxx - minx < kSmallExtent && maxy - miny < kSmallExtent &&
-                       (uint32_t)((qx1 - qx0 + 1) * (qy1 - qy0 + 1)) <= Q.small_area;
+                       fast_size((uint32_t)(qx1 - qx0 + 1), (uint32_t)(qy1 - qy0 + 1), Q);
     return small ? kFast : kSlowSetup;
 }
 
@@ -544,10 +554,21 @@ __device__ __forceinline__ unsigned long long fragment(float pa, float pb, float
     return ((unsigned long long)__float_as_uint(z) << 32) | (unsigned long long)(id + 1u);
 }
 
+// The sample of pixel (lx, ly) of a record's bbox.
+__device__ __forceinline__ void draw_sample(const TriRec& r, uint32_t lx, uint32_t ly, uint32_t d, const RasterCtx& c) {
+    SmallEdges e;
+    edges_at(e, (int32_t)(int16_t)(r.v[0] & 0xFFFFu), (int32_t)r.v[0] >> 16, (int32_t)(int16_t)(r.v[1] & 0xFFFFu),
+             (int32_t)r.v[1] >> 16, (int32_t)(int16_t)(r.v[2] & 0xFFFFu), (int32_t)r.v[2] >> 16, (r.bits >> 7) & 7u,
+             (int32_t)(lx << 8) + 128, (int32_t)(ly << 8) + 128);
+    if ((e.e0 | e.e1 | e.e2) >= 0)
+        plot(c.depth + (size_t)((r.origin >> 16) + ly) * c.w + (r.origin & 0xFFFFu) + lx,
+             fragment(r.pa, r.pb, r.z0, e.fx, e.fy, (d << 7) | (r.bits & 127u)));
+}
+
 // Second stage of the fast instance: up to 32 compacted candidates, one
 // per lane (ct = meshlet-local triangle index, 0xffffffff = none).  A
-// candidate that is back-facing or of zero area is dropped; one whose bbox
-// exceeds small_area pixels or whose extent leaves int32 edge values needs
+// candidate that is back-facing or of zero area is dropped; one that is not of
+// a fast_size or whose extent leaves int32 edge values needs
 // the slow instance (the return value); the rest are set up and
 // rasterised.  A triangle whose
 // clamped bbox has at most kLaneArea pixels is rasterised by its own lane;
@@ -578,7 +599,7 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
         const int32_t px0 = max((minx - 128 + 255) >> 8, 0), px1 = min((maxx - 128) >> 8, (int32_t)c.w - 1);
         const int32_t py0 = max((miny - 128 + 255) >> 8, 0), py1 = min((maxy - 128) >> 8, (int32_t)c.h - 1);
         const uint32_t bw = (uint32_t)(px1 - px0 + 1), bh = (uint32_t)(py1 - py0 + 1);
-        const bool live = !back && fits && A != 0 && bw * bh <= Q.small_area;
+        const bool live = !back && fits && A != 0 && fast_size(bw, bh, Q);
         if (!back && !live) {
             const int64_t A64 = (int64_t)(q1.x - q0.x) * (q2.y - q0.y) - (int64_t)(q1.y - q0.y) * (q2.x - q0.x);
             slow = A64 != 0;
@@ -670,6 +691,19 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
                 report(Q.status, kStatusQueueOverflow, slot);
             }
         }
+        // what a full queue refused above small_area, one after another
+        unsigned refused = __ballot_sync(0xffffffffu, coop_area > Q.small_area);
+        for (; refused; refused &= refused - 1u) {
+            const int from = __ffs(refused) - 1;
+            if (lane == from) recs[0] = rec;
+            const uint32_t area = __shfl_sync(0xffffffffu, coop_area, from);
+            if (lane == from) coop_area = 0;
+            __syncwarp();
+            const TriRec r = recs[0];
+            const uint32_t bw = (r.bits >> 10) & 127u;
+            for (uint32_t p = lane; p < area; p += 32) draw_sample(r, p % bw, p / bw, d, c);
+            __syncwarp();
+        }
         coop = __ballot_sync(0xffffffffu, coop_area != 0);
         if (coop == 0) return slow;
     }
@@ -702,13 +736,7 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
             const TriRec r = recs[j];
             const uint32_t local = p - starts[j], bw = (r.bits >> 10) & 127u;
             const uint32_t ly = (local * (r.bits >> 17)) >> 12, lx = local - ly * bw;
-            SmallEdges e;
-            edges_at(e, (int32_t)(int16_t)(r.v[0] & 0xFFFFu), (int32_t)r.v[0] >> 16, (int32_t)(int16_t)(r.v[1] & 0xFFFFu),
-                     (int32_t)r.v[1] >> 16, (int32_t)(int16_t)(r.v[2] & 0xFFFFu), (int32_t)r.v[2] >> 16,
-                     (r.bits >> 7) & 7u, (int32_t)(lx << 8) + 128, (int32_t)(ly << 8) + 128);
-            if ((e.e0 | e.e1 | e.e2) >= 0)
-                plot(c.depth + (size_t)((r.origin >> 16) + ly) * c.w + (r.origin & 0xFFFFu) + lx,
-                     fragment(r.pa, r.pb, r.z0, e.fx, e.fy, (d << 7) | (r.bits & 127u)));
+            draw_sample(r, lx, ly, d, c);
         }
     }
     __syncwarp();
