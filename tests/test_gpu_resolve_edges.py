@@ -79,3 +79,22 @@ def test_repeated_textures_match_oracle(renderer, size, offset, scale):
     assert np.array_equal(ids, exp["ids"])
     close, off = U.rgba_close(rgba, exp["rgba"])
     assert close, f"{off} pixels differ"
+
+
+@pytest.mark.parametrize("extra", [-1, 1])
+def test_views_about_the_pixels_per_thread_line(renderer, extra):
+    """A view just below and one just above the size from which a resolve
+    thread takes four pixels."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    h = 1301
+    w = 20 * 1024 * sms // h + extra
+    assert (w * h >= 20 * 1024 * sms) == (extra > 0)
+    host = U.small_grid()
+    dev = DeviceScene(host, "cuda")
+    cam = scene.camera(*CAM, (0, 1, 0), 70.0, w / h)
+    v = U.ViewBuffers.allocate(w, h, cam, host.draw_count)
+    renderer.frame(dev, [v], FLAGS)
+    exp = ob.frame(ob.OracleScene(host), cam, w, h, U.oracle_flags(FLAGS))
+    assert np.array_equal(U.u32(v.visbuffer), exp["ids"])
+    close, off = U.rgba_close(U.u32(v.color), exp["rgba"])
+    assert close, f"{off} pixels differ"

@@ -669,7 +669,12 @@ void launch_resolve(const SceneArgs& S, const DeviceView* views, uint32_t nviews
         if (done) return;
     }
     const uint64_t px = (uint64_t)max_w * max_h;
-    uint32_t bx = (uint32_t)((px + 511) / 512);
+    // Two pixels a thread, and four where that still leaves 20 CTAs per SM: the
+    // torus grid at 4K 533 -> 524.5 us a frame, at 2560x1440 349 -> 344, but at
+    // 1080p 268 -> 271.5 (its last wave) and for the flat resolve of a sphere at
+    // 2560x1440 43.2 -> 44.0; six and eight a thread gain no more.
+    const uint32_t each = (tex || mv) && px >= 20ull * 1024 * sm_count ? 1024u : 512u;
+    uint32_t bx = (uint32_t)((px + each - 1) / each);
     if (bx > 65535u) bx = 65535u;
     dim3 grid(bx, nviews);
     if (tex && mv)
