@@ -239,7 +239,7 @@ __host__ __device__ __forceinline__ uint64_t mip_offset(uint32_t w0, uint32_t h0
     return off;
 }
 
-// HiZ tiling (single-pass reduce): a CTA owns an 8x8 tile of the highest
+// HiZ tiling: a CTA owns an 8x8 tile of the highest
 // tiled level (at most level 4) and the matching 2^k-times larger tiles of
 // the levels below it.  Levels with a zero dimension are never tiled.
 constexpr int kHizTileLevels = 4;

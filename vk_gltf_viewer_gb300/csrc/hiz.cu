@@ -1,5 +1,6 @@
 // HiZ min-pyramid: the reduce chain of application.cpp:951-1003 that runs
-// shaders/hiz_reduce.comp.glsl once per level, here in one launch per frame.
+// shaders/hiz_reduce.comp.glsl once per level, here in one launch per reduce, or
+// two for large views (hiz_second).
 //
 // Level i (1..L) writes mip i-1 at size (W>>i, H>>i) from mip i-2 (the depth
 // image for i = 1): texel p = MIN over the bilinear footprint of the source
@@ -11,14 +12,15 @@
 // pos == size through, whose image store is out of bounds; only pos < size is
 // written here.
 //
-// Single pass: each CTA owns a 4x4 tile of level 4 and the 8x8, 16x16 and
+// Each CTA owns a 4x4 tile of level 4 and the 8x8, 16x16 and
 // 32x32 tiles of levels 3, 2, 1 above it (510 CTAs of 256 threads at
 // 1920x1080, several resident per SM).  For odd sizes the footprints do
 // not nest, so each CTA computes the hull of its owned tile and the
 // footprint of the level above it (a halo of a few texels, recomputed rather
 // than exchanged), keeping levels 1-3 in shared memory and reading the depth
-// image once.  The last CTA of a view to finish computes the remaining top
-// levels: the footprints of all their columns and rows in one table, the
+// image once.  The remaining top levels are the second launch's, tiled in the
+// same way from level 4, or, for smaller views, the last CTA's of a view to
+// finish: the footprints of all their columns and rows in one table, the
 // first of them from the top tiled mip in L2, the rest from shared memory
 // with one barrier per level.
 #include <atomic>

@@ -193,7 +193,7 @@ void launch_world_transforms(const WorldArgs& W, float time, float* transforms, 
 // k_world_draws: the MeshletDraw list as 3 words per draw.
 void launch_world_draws(const WorldArgs& W, uint32_t* draws, uint32_t sm_count, cudaStream_t stream);
 
-// k_decode_bc: BC1-BC5 blocks -> RGBA8, one thread per texel.
+// k_decode_bc: BC1-BC5 and BC7 blocks -> RGBA8, one thread per block.
 // Sample planes of a JPEG (8-bit, pitch bytes per row) for the colour
 // conversion; rx / ry = hmax / h, vmax / v of each component.
 struct JpegPlanes {

@@ -7,9 +7,9 @@
 // vertices into shared memory, then each lane sets up one triangle at a time
 // (homogeneous backface determinant, outcode reject, near/far and guard-band
 // clipping, 28.8 fixed-point snap, top-left edge functions, depth plane).
-// Small triangles are rasterised by the lane itself; larger ones are cut into
-// chunk x chunk pixel rectangles and binned into a queue that a second
-// kernel drains with one warp per rectangle.  Every covered sample performs a
+// Triangles of a few pixels are rasterised by the lane itself or by its warp;
+// larger ones go to a queue, as one rectangle or cut into chunk x chunk pixel
+// rectangles, that k_raster_big drains with a warp per rectangle.  Every covered sample performs a
 // 64-bit max of (depth bits << 32 | id + 1), which is the order-independent
 // form of the GREATER_OR_EQUAL depth test with ties won by the later draw.
 #include <atomic>
@@ -744,8 +744,7 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
 }
 
 // Warp-per-meshlet raster.  The fast instance (SLOW = false) handles every
-// triangle that needs no clipping and fits the cooperative small-triangle
-// path, and appends a meshlet that has any other triangle to the view's
+// triangle that needs no clipping and is of a fast_size, and appends a meshlet that has any other triangle to the view's
 // deferred list.  The slow instance (SLOW = true) re-runs those meshlets and
 // handles only the remaining triangles (homogeneous clipping, large or
 // off-screen-spanning triangles), so the fast instance calls no function.

@@ -373,7 +373,7 @@ __device__ void shade_textured(const SceneArgs& S, const Frag& f, float out[4]) 
 // Only the x, y and w rows of prevViewProjection * M are needed; each
 // vertex's previous clip position is folded into the interpolation sums
 // ((l0 p0 + l1 p1) + l2 p2) as it is computed, which keeps the variant small
-// enough for six CTAs per SM.
+// enough for five CTAs per SM.
 __device__ uint32_t motion_vector(const SceneArgs& S, const DeviceView& V, const Frag& f) {
     float rx[4], ry[4], rw[4];  // rows x, y, w of prev_view_projection * M (per column)
     if (V.prev_mvps && f.transform_index < S.transform_count) {
