@@ -743,6 +743,30 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
     return slow;
 }
 
+// A warp's shared memory, in one piece: one base register addresses all of it
+// (with an array of each member per CTA the fast instance spilled 34 bytes of
+// its 72 registers, with this 30, in colder places: 256 views of the torus grid
+// 30.43 -> 29.39 ms, of 128^2 1,380 -> 1,328 us, the 4K frame 515.2 -> 506.3, 1080p
+// 252.4 -> 248.6).
+struct __align__(16) WarpShared {
+    // per vertex: clip {x, y, z, w} (slow instance) or clip {x, y, w} and the
+    // snapped depth (fast instance); the snapped {X, Y} (28.8)
+    float4 clip[64];
+    TriRec tri[32];
+    int2 xy[64];
+    uint32_t idx[96];           // the meshlet's triangle-index bytes (<= 126 triangles)
+    float mvp[16];
+    // Per-meshlet headers of the current run, resolved one item per lane so
+    // that the dependent loads (list entry -> draw -> primitive -> meshlet
+    // record, material) of up to kMaxRun meshlets are in flight together instead
+    // of one meshlet after another.
+    ItemHeader hdr[kMaxRun];
+    RasterCtx ctx;
+    float tdet;
+    uint16_t start[32];
+    uint8_t ring[128];          // the compacted candidate triangle indices (fast instance)
+};
+
 // Warp-per-meshlet raster.  The fast instance (SLOW = false) handles every
 // triangle that needs no clipping and is of a fast_size, and appends a meshlet that has any other triangle to the view's
 // deferred list.  The slow instance (SLOW = true) re-runs those meshlets and
@@ -751,18 +775,7 @@ __device__ __forceinline__ bool raster_small(uint32_t ct, const uint8_t* sidx8, 
 template <int WARPS, bool SLOW>
 __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER_SM) / WARPS) k_raster(RasterParams P) {
     pdl_begin();
-    // per vertex: clip {x, y, z, w} (slow instance) or clip {x, y, w} and the
-    // snapped depth (fast instance); the snapped {X, Y} (28.8)
-    __shared__ float4 s_clip[WARPS][64];
-    __shared__ int2 s_xy[WARPS][64];
-    // the meshlet's triangle-index bytes (<= 126 triangles)
-    __shared__ uint32_t s_idx[WARPS][96];
-    __shared__ TriRec s_tri[WARPS][32];
-    // the compacted candidate triangle indices (fast instance)
-    __shared__ uint8_t s_ring[WARPS][128];
-    __shared__ uint16_t s_start[WARPS][32];
-    __shared__ float s_mvp[WARPS][16];
-    __shared__ float s_tdet[WARPS];
+    __shared__ WarpShared s_warp[WARPS];
     // exclusive prefix of the views' work counts: view v owns the global
     // work items [s_pre[v], s_pre[v + 1])
     // (sized by the launch: 18 KB a CTA leave seven of them in 132 KB and the
@@ -820,32 +833,27 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
     if (total == 0) return;
     const uint32_t slot = P.lists.deferred_slot;
     const uint32_t defer_cap = P.deferred_cap;
-    float4* clip = s_clip[warp];
-    int2* sxy = s_xy[warp];
+    WarpShared& W = s_warp[warp];
+    float4* clip = W.clip;
+    int2* sxy = W.xy;
     // {depth bits, flags} of every vertex, which the fast instance reads only
     // for a meshlet that is not entirely inside the view volume, before it
     // writes a record
-    static_assert(sizeof(s_tri[0]) >= 64 * sizeof(int2), "vertex flags share the records' memory");
-    int2* szf = reinterpret_cast<int2*>(s_tri[warp]);
-    uint32_t* sidx = s_idx[warp];
+    static_assert(sizeof(W.tri) >= 64 * sizeof(int2), "vertex flags share the records' memory");
+    int2* szf = reinterpret_cast<int2*>(W.tri);
+    uint32_t* sidx = W.idx;
     const uint8_t* sidx8 = reinterpret_cast<const uint8_t*>(sidx);
-    TriRec* recs = s_tri[warp];
-    uint16_t* starts = s_start[warp];
+    TriRec* recs = W.tri;
+    uint16_t* starts = W.start;
     // Warps take runs of `grab` consecutive work items, their own first and
     // then from one counter, so views are drawn roughly in order (their depth buffers stay in L2) and
     // no warp idles while work is left.
     const uint32_t warps_total = gridDim.x * WARPS;
     const uint32_t grab = max(1u, min(kMaxRun, total / (warps_total * 8u)));
-    uint32_t cur_v = 0xffffffffu, cur_t = 0xffffffffu;  // view and node of s_mvp
+    uint32_t cur_v = 0xffffffffu, cur_t = 0xffffffffu;  // view and node of W.mvp
     const DeviceView* Vp = P.views;
-    __shared__ RasterCtx s_ctx[WARPS];
-    RasterCtx& c = s_ctx[warp];
-    // Per-meshlet headers of the current run, resolved one item per lane so
-    // that the dependent loads (list entry -> draw -> primitive -> meshlet
-    // record, material) of up to kMaxRun meshlets are in flight together instead
-    // of one meshlet after another.
-    __shared__ ItemHeader s_hdr[WARPS][kMaxRun];
-    ItemHeader* hdr = s_hdr[warp];
+    RasterCtx& c = W.ctx;
+    ItemHeader* hdr = W.hdr;
     // the next run is requested while the current one is drawn, so the
     // atomic's round trip is off the critical path
     // The first run of each warp is its own, a warp of every CTA before the
@@ -961,25 +969,25 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
             cur_t = transform_index;
             if (same_node) {
             } else if (lane < 16 && V.mvps && transform_index < P.S.transform_count) {
-                s_mvp[warp][lane] = __ldg(V.mvps + 16 * (size_t)transform_index + lane);
+                W.mvp[lane] = __ldg(V.mvps + 16 * (size_t)transform_index + lane);
             } else if (lane < 16) {
                 const int cc = lane >> 2, j = lane & 3;
                 const float4 mc = __ldg(reinterpret_cast<const float4*>(Mg) + cc);
                 const float* vp = V.cam->view_projection;
-                s_mvp[warp][lane] = fadd(fadd(fadd(fmul(vp[0 * 4 + j], mc.x), fmul(vp[1 * 4 + j], mc.y)),
+                W.mvp[lane] = fadd(fadd(fadd(fmul(vp[0 * 4 + j], mc.x), fmul(vp[1 * 4 + j], mc.y)),
                                               fmul(vp[2 * 4 + j], mc.z)),
                                          fmul(vp[3 * 4 + j], mc.w));
             } else if (lane == 16 && have_tdet) {
-                s_tdet[warp] = P.S.tdets[transform_index];
+                W.tdet = P.S.tdets[transform_index];
             } else if (lane == 16) {
                 float M[16];
     #pragma unroll
                 for (int q = 0; q < 16; ++q) M[q] = __ldg(Mg + q);
-                s_tdet[warp] = det4(M);
+                W.tdet = det4(M);
             }
             if (!same_node) __syncwarp();
-            const float tdet = s_tdet[warp];
-            const float* mvp = s_mvp[warp];
+            const float tdet = W.tdet;
+            const float* mvp = W.mvp;
             // Vertex stage: clip position, outcode, guard flag and the 28.8 snap,
             // each computed once per meshlet vertex (two per lane).  All global
             // loads of the stage, and the triangle-index words (32-bit loads
@@ -1078,7 +1086,7 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
                 // backface, area and size tests, the setup and the raster run
                 // on full warps (at most about a quarter of the triangles of
                 // a dense meshlet have a sample in their bbox).
-                uint8_t* ring = s_ring[warp];
+                uint8_t* ring = W.ring;
                 uint32_t pending = 0;
                 for (uint32_t tbase = H.t0; tbase < tc; tbase += 32) {
                     const uint32_t t = tbase + lane;
