@@ -435,8 +435,8 @@ int vkgv_create(const vkgv_config* config, vkgv_ctx** out_ctx) {
         delete ctx;
         return VKGV_INVALID_ARG;
     }
-    uint32_t mpc = ctx->cfg.meshlets_per_cta ? ctx->cfg.meshlets_per_cta : 4;
-    if (mpc != 1 && mpc != 2 && mpc != 4 && mpc != 8) {
+    const uint32_t mpc = ctx->cfg.meshlets_per_cta;  // 0: by the launch's size
+    if (mpc != 0 && mpc != 1 && mpc != 2 && mpc != 4 && mpc != 8) {
         delete ctx;
         return VKGV_INVALID_ARG;
     }

@@ -1235,14 +1235,14 @@ uint32_t raster_split(uint32_t sm_count) { return sm_count * VKGV_RASTER_SPLIT_P
 
 // One wave of CTAs: every warp stays resident and takes work until none is
 // left.
-template <int WARPS>
+template <int WARPS, int SLOW_WARPS = WARPS>
 void launch_variant(RasterParams P, uint32_t sm_count, uint32_t blocks_override, cudaStream_t stream) {
     const uint32_t fast = blocks_override ? blocks_override : sm_count * (VKGV_RASTER_WARPS_PER_SM / WARPS);
-    const uint32_t slow = blocks_override ? blocks_override : sm_count * (16 / WARPS > 0 ? 16 / WARPS : 1);
+    const uint32_t slow = blocks_override ? blocks_override : sm_count * (16 / SLOW_WARPS > 0 ? 16 / SLOW_WARPS : 1);
     P.split = raster_split(sm_count);
     const size_t pre = sizeof(uint32_t) * (P.nviews + 1);
     launch_pdl(k_raster<WARPS, false>, dim3(fast), dim3(WARPS * 32), pre, stream, P);
-    launch_pdl(k_raster<WARPS, true>, dim3(slow), dim3(WARPS * 32), pre, stream, P);
+    launch_pdl(k_raster<SLOW_WARPS, true>, dim3(slow), dim3(SLOW_WARPS * 32), pre, stream, P);
 }
 
 }  // namespace
@@ -1271,6 +1271,17 @@ void launch_raster(const SceneArgs& S, const DeviceView* views, uint32_t nviews,
         P.views = views + v0;
         P.nviews = nviews - v0 < kRasterMaxViews ? nviews - v0 : kRasterMaxViews;
         P.view_base = v0;
+        // One warp a CTA addresses its shared memory by constants and spills
+        // nothing (256 views of the torus grid 29.41 -> 28.77 ms, the 4K frame
+        // 506.5 -> 495.1 us, 1080p 248.8 -> 242.6), but a launch of few meshlets
+        // waits for its 4,256 CTAs (84 meshlets: 29.2 -> 32.0 us; 1,152: 30.1 ->
+        // 30.4; 64 views of 290: 554.8 -> 551.2), and above 512 views their
+        // prefixes leave no room for 28 of them on an SM.  The slow instance
+        // keeps four (1080p 244.1 with one).
+        if (!cfg.warps_per_cta && (uint64_t)S.draw_count * P.nviews >= 16384 && P.nviews <= 512) {
+            launch_variant<1, 4>(P, sm_count, cfg.blocks_per_view, stream);
+            continue;
+        }
         switch (cfg.warps_per_cta) {
             case 1: launch_variant<1>(P, sm_count, cfg.blocks_per_view, stream); break;
             case 2: launch_variant<2>(P, sm_count, cfg.blocks_per_view, stream); break;
