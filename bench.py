@@ -493,7 +493,7 @@ def run_world(r, host, local, args, stream, peak):
                            "frac": achieved / peak, "algorithmic_bytes": draw_bytes,
                            "note": "12 B per draw written + 8 B per (primitive, slot) segment and its offset read; "
                                    "50 launches per CUDA graph, so the 10 MB list stays L2-resident"},
-        "gpu_launches_per_update": 2, "gpu_launches_per_draw_build": 1,
+        "gpu_launches_per_update": 1, "gpu_launches_per_draw_build": 1,
         "device_status": list(status),
     }
     # the same scene as a .glb (1 primitive, 2,057 nodes, 1,098 channels)
