@@ -1018,12 +1018,15 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
             m4v(mvp, xy0.x, xy0.y, zz0, 1.0f, &cv[0].x);
             m4v(mvp, xy1.x, xy1.y, zz1, 1.0f, &cv[1].x);
             // Inside the view volume no outcode, guard or snap-range test can
-            // fire: a meshlet with all vertices inside skips them here and in
+            // fire, if w and its reciprocal are finite and not subnormal (an
+            // infinite w passes the volume's comparisons, and snaps to no
+            // place): a meshlet with all vertices inside skips them here and in
             // the pre-filter (issue-bound: 256 views of 128^2 1,731 -> 1,474 us
             // a frame, the 256-view torus grid 37.0 -> 32.2 ms, with the
             // pre-filter on 8-byte vertices and the relative edge setup).
             auto inside = [](const float4& q) {
-                return fabsf(q.x) <= q.w && fabsf(q.y) <= q.w && q.z >= 0.0f && q.z <= q.w && q.w > 0.0f;
+                return fabsf(q.x) <= q.w && fabsf(q.y) <= q.w && q.z >= 0.0f && q.z <= q.w && q.w >= 0x1p-100f &&
+                       q.w <= 0x1p100f;
             };
             const bool plain = !SLOW && __all_sync(0xffffffffu, (!h0 || inside(cv[0])) && (!h1 || inside(cv[1])));
 #pragma unroll
