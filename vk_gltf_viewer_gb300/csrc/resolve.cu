@@ -301,6 +301,18 @@ __device__ void frag_setup(const SceneArgs& S, const DeviceView& V, uint32_t px,
     }
 }
 
+// A material's base colour factor, in one 16-byte load where the array allows
+// it.
+__device__ __forceinline__ void load_albedo(const SceneArgs& S, const vkgv_material* p, float out[4]) {
+    if ((reinterpret_cast<uintptr_t>(S.mats) & 15u) == 0) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(p));
+        out[0] = a.x, out[1] = a.y, out[2] = a.z, out[3] = a.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) out[k] = __ldg(p->albedo_factor + k);
+    }
+}
+
 // The shading fields of a material, in 16-byte loads where the array allows
 // them (a record is 48 bytes).
 __device__ __forceinline__ vkgv_material load_material(const SceneArgs& S, const vkgv_material* p) {
@@ -446,14 +458,11 @@ __device__ __forceinline__ void resolve_pixel(const SceneArgs& S, const DeviceVi
             if (TEXTURED) {
                 shade_textured(S, f, lin);
             } else {
-                const float4 a = *reinterpret_cast<const float4*>(f.mat->albedo_factor);
-                lin[0] = a.x, lin[1] = a.y, lin[2] = a.z, lin[3] = a.w;
+                load_albedo(S, f.mat, lin);
             }
         } else {
             const vkgv_meshlet_draw dr = S.draws[id >> VKGV_TRIANGLE_BITS];
-            const vkgv_material& mat = S.mats[S.prims[dr.primitive_index].material_index];
-            const float4 a = *reinterpret_cast<const float4*>(mat.albedo_factor);
-            lin[0] = a.x, lin[1] = a.y, lin[2] = a.z, lin[3] = a.w;
+            load_albedo(S, S.mats + S.prims[dr.primitive_index].material_index, lin);
         }
         if (rgba) out = TEXTURED ? pack_rgba_fast(lin) : pack_rgba(lin);
     }
