@@ -236,6 +236,7 @@ int build_views(vkgv_ctx* ctx, const vkgv_scene* scene, const vkgv_view* views, 
     P.S.primitive_count = scene->cone_table ? scene->primitive_count : 0;
     P.S.transform_count = scene->transform_count;
     P.S.tdets = nullptr;
+    P.hiz.line = hiz_line(n);
     for (uint32_t i = 0; i < n; ++i) {
         const vkgv_view& v = views[i];
         rc = validate_view(ctx, v, flags);

@@ -239,9 +239,9 @@ __host__ __device__ __forceinline__ uint64_t mip_offset(uint32_t w0, uint32_t h0
     return off;
 }
 
-// HiZ tiling: a CTA owns an 8x8 tile of the highest
-// tiled level (at most level 4) and the matching 2^k-times larger tiles of
-// the levels below it.  Levels with a zero dimension are never tiled.
+// HiZ tiling: a CTA owns a 4x4 tile of the highest tiled level (at most level
+// 4) and the matching 2^k-times larger tiles of the levels below it.  Levels
+// with a zero dimension are never tiled.
 constexpr int kHizTileLevels = 4;
 constexpr int kHizTopTile = 4;
 
@@ -253,14 +253,24 @@ __host__ __device__ __forceinline__ int hiz_tile_levels(uint32_t w, uint32_t h, 
 
 // Whether a view's levels above the four tiled ones are reduced by a second
 // launch, tiled in the same way from level 4, instead of by the last CTA of
-// the first one: from 2,048 texels in level 5 on.  The second launch takes 14 us
-// at any size, the last CTA 9 us at 1920x1080 (1,980 texels; 277.5 against 285.9
-// us a frame) but 30 us at 3840x2160, in 43 KB of shared memory that also kept
-// the resolve from running beside it (637 -> 537 us a frame).
-__host__ __device__ __forceinline__ bool hiz_second(uint32_t w, uint32_t h, uint32_t levels) {
+// the first one: from `line` texels in level 5 on (hiz_line).
+__host__ __device__ __forceinline__ bool hiz_second(uint32_t w, uint32_t h, uint32_t levels, uint32_t line) {
     return hiz_tile_levels(w, h, levels) == kHizTileLevels && levels > (uint32_t)kHizTileLevels &&
-           (w >> (kHizTileLevels + 1)) * (h >> (kHizTileLevels + 1)) >= 2048u;
+           (w >> (kHizTileLevels + 1)) * (h >> (kHizTileLevels + 1)) >= line;
 }
+
+// The second launch takes some 14 us at any size and for any number of views,
+// the last CTA 9 us for 1,980 texels (1920x1080) and 30 us for 8,040
+// (3840x2160), in shared memory that grows with them and keeps a resolve from
+// running beside it.  Frames of one view, last CTA -> second launch: 1080p torus
+// grid 277.5 -> 285.9 us; two passes of a sphere at 2304x1296 (2,880 texels) 77.6
+// -> 84.7, at 2880x1620 (4,500) 95.5 -> 100.1, torus grid seen from inside at
+// 2560x1440 (3,600) 311.5 -> 309.2; at 3200x1800 (5,600) the sphere 107.4 -> 109.5,
+// without a resolve 69.2 -> 65.0, the torus grid 412.9 -> 405.5; at 3840x2160 141.6
+// -> 132.3 and 552.9 -> 505.0.  Frames of several views share the launch: two
+// spheres of 2048x1100 (2,176) 101.9 -> 101.1, of 2560x1440 132.1 -> 129.1, two
+// torus grids of 2048x1100 1,467 -> 1,443, 16 spheres of it 351.8 -> 343.6.
+inline uint32_t hiz_line(uint32_t nviews) { return nviews == 1 ? 5120u : 2048u; }
 
 __host__ __device__ __forceinline__ int hiz_tile_edge(int level, int top) { return kHizTopTile << (top - level); }
 

@@ -114,11 +114,11 @@ __device__ __forceinline__ float reduce_texel(int x, int y, uint32_t dw, uint32_
 // the same one on a smaller view.
 template <bool FIRST>
 __global__ void __launch_bounds__(kThreads, 5) k_hiz(const DeviceView* __restrict__ views, uint32_t* status,
-                                                  uint32_t tail) {
+                                                  uint32_t tail, uint32_t line) {
     pdl_begin();
     const DeviceView& V = views[blockIdx.z];
     if (!V.pyr || V.pyr_levels == 0) return;
-    const bool second = hiz_second(V.w, V.h, V.pyr_levels);
+    const bool second = hiz_second(V.w, V.h, V.pyr_levels, line);
     if (!FIRST && !second) return;
     constexpr uint32_t kSkip = FIRST ? 0u : (uint32_t)kHizTileLevels;
     const uint32_t w = V.w >> kSkip, h = V.h >> kSkip, L = V.pyr_levels - kSkip;
@@ -387,7 +387,7 @@ uint32_t tail_floats(uint32_t w, uint32_t h, uint32_t levels) {
 
 template <bool FIRST>
 void launch_pass(const DeviceView* views, uint32_t nviews, uint32_t tiles_x, uint32_t tiles_y, uint32_t tail,
-                 uint32_t* status, cudaStream_t stream) {
+                 uint32_t line, uint32_t* status, cudaStream_t stream) {
     // The dynamic shared-memory limit is a per-device function attribute:
     // set it once for each device a launch runs on (setting it twice is
     // harmless, so concurrent first launches need no lock).
@@ -403,7 +403,7 @@ void launch_pass(const DeviceView* views, uint32_t nviews, uint32_t tiles_x, uin
     if (tail > (uint32_t)kTailMax) tail = 0;
     const uint32_t floats = tail > (uint32_t)kTileFloats ? tail : (uint32_t)kTileFloats;
     dim3 grid(tiles_x ? tiles_x : 1, tiles_y ? tiles_y : 1, nviews);
-    launch_pdl(k_hiz<FIRST>, grid, dim3(kThreads), floats * sizeof(float), stream, views, status, tail);
+    launch_pdl(k_hiz<FIRST>, grid, dim3(kThreads), floats * sizeof(float), stream, views, status, tail, line);
 }
 
 }  // namespace
@@ -416,7 +416,7 @@ void hiz_add_view(HizShape& shape, uint32_t w, uint32_t h, uint32_t levels) {
         ty = y > ty ? y : ty;
     };
     widen(shape.tiles_x, shape.tiles_y, w, h, levels);
-    if (hiz_second(w, h, levels)) {
+    if (hiz_second(w, h, levels, shape.line)) {
         w >>= kHizTileLevels, h >>= kHizTileLevels, levels -= kHizTileLevels;
         widen(shape.tiles_x2, shape.tiles_y2, w, h, levels);
         const uint32_t t = tail_floats(w, h, levels);
@@ -429,9 +429,9 @@ void hiz_add_view(HizShape& shape, uint32_t w, uint32_t h, uint32_t levels) {
 
 void launch_hiz(const DeviceView* views, uint32_t nviews, const HizShape& shape, uint32_t* status,
                 cudaStream_t stream) {
-    launch_pass<true>(views, nviews, shape.tiles_x, shape.tiles_y, shape.tail, status, stream);
+    launch_pass<true>(views, nviews, shape.tiles_x, shape.tiles_y, shape.tail, shape.line, status, stream);
     if (shape.tiles_x2)
-        launch_pass<false>(views, nviews, shape.tiles_x2, shape.tiles_y2, shape.tail2, status, stream);
+        launch_pass<false>(views, nviews, shape.tiles_x2, shape.tiles_y2, shape.tail2, shape.line, status, stream);
 }
 
 }  // namespace vkgv

@@ -65,6 +65,7 @@ void launch_raster(const SceneArgs& S, const DeviceView* views, uint32_t nviews,
 // (shared memory of the last CTA's levels) of its first launch and, where a
 // view needs one (tiles_x2 > 0), of its second.
 struct HizShape {
+    uint32_t line = 0;  // hiz_line of the number of views
     uint32_t tiles_x = 1, tiles_y = 1, tail = 0;
     uint32_t tiles_x2 = 0, tiles_y2 = 0, tail2 = 0;
 };
