@@ -825,6 +825,7 @@ int vkgv_world_create(vkgv_ctx* ctx, const vkgv_world_desc* desc, vkgv_world** o
     A.seg_count = P.seg_count;
     A.draw_count = (uint32_t)P.draw_count;
     A.max_chain = P.max_chain;
+    A.repeated = P.repeated;
     w->draw_count = P.draw_count;
     *out_world = w;
     return VKGV_OK;

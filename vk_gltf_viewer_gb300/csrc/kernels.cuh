@@ -167,6 +167,7 @@ struct WorldArgs {
     uint32_t draw_count;
     uint32_t tile_count;
     uint32_t max_chain;             // nodes on the longest path
+    uint64_t repeated;              // channels that a lane per node of every path samples again
 };
 
 constexpr uint32_t kWorldTile = 1024;    // draws per k_world_draws block
@@ -184,7 +185,7 @@ struct WorldPlan {
     std::vector<uint2> seg_info;
     std::vector<uint32_t> tile_seg;
     uint32_t node_count = 0, slot_count = 0, seg_count = 0, max_chain = 0;
-    uint64_t draw_count = 0;
+    uint64_t draw_count = 0, repeated = 0;
 };
 
 // Validates a world description and walks its tree; returns a vkgv_status.

@@ -324,10 +324,16 @@ void launch_slots(const WorldArgs& W, float time, float* transforms, cudaStream_
 // lane per node pays (524,288 nodes, meshes on the leaves of paths of 4 or 8:
 // 17.3 and 26.3 us, two launches 30.2 and 31.6), for paths of two also two
 // (24.3 us, 32.1), but not four (meshes on all nodes of paths of 4: 57 us, 33).
+// Sampling is what the lanes do most of where nodes have many channels, so the
+// channels sampled again are counted too (trees of 32,581 slots, paths of 3, 1 / 2
+// / 10 animations of 3 channels a node, 0.19 / 0.39 / 1.95 million again: two
+// launches 9.0, 11.6, 32.0 us, this 9.3, 13.6, 46.5; 32,768 slots, paths of 2, 1 / 2 /
+// 50 animations, 0.10 / 0.20 / 4.9 million: 8.8, 11.4, 138 us, this 7.9, 11.5, 187).
 void launch_world_transforms(const WorldArgs& W, float time, float* transforms, cudaStream_t stream) {
     const uint32_t group = W.max_chain <= 1 ? 1 : W.max_chain <= 2 ? 2 : W.max_chain <= 4 ? 4 : 8;
     const uint64_t lanes = (uint64_t)W.slot_count * group;
-    if (W.max_chain <= group && lanes <= std::max<uint64_t>(131072, (uint64_t)W.node_count * (group == 2 ? 2 : 1))) {
+    if (W.max_chain <= group && W.repeated <= 196608 &&
+        lanes <= std::max<uint64_t>(131072, (uint64_t)W.node_count * (group == 2 ? 2 : 1))) {
         if (!lanes) return;
         if (group == 1) launch_slots<1>(W, time, transforms, stream);
         else if (group == 2) launch_slots<2>(W, time, transforms, stream);
@@ -500,6 +506,9 @@ int plan_world(const vkgv_world_desc& D, WorldPlan& P, std::string& err) {
         while (s + 1 < P.seg_info.size() && P.seg_first[s + 1] <= d) ++s;
         P.tile_seg[t] = (uint32_t)s;
     }
+    uint64_t sampled = 0;
+    for (uint32_t n : P.chain_nodes) sampled += P.chan_offsets[n + 1] - P.chan_offsets[n];
+    P.repeated = sampled > P.chans.size() ? sampled - P.chans.size() : 0;
     P.node_count = N;
     P.slot_count = (uint32_t)(P.chain_offsets.size() - 1);
     P.seg_count = (uint32_t)P.seg_info.size();
