@@ -3,9 +3,10 @@ meshlets per CTA {1, 2, 4} for a workload on this GPU.
 
 The sweep itself is native (vkgv_autotune: one context and one captured
 frame graph per candidate, timed with CUDA events).  Results are cached in a
-JSON file keyed by GPU name, SM count and a workload key (triangles, draws,
-flags, view count and resolutions), so a workload is swept once per GPU
-model.  The cache path is $VKGV_AUTOTUNE_CACHE, else
+JSON file keyed by GPU name, SM count, the native library's contents and a
+workload key (triangles, draws, flags, view count and resolutions), so a
+workload is swept once per GPU model and build: another build's kernels may
+want another shape.  The cache path is $VKGV_AUTOTUNE_CACHE, else
 ~/.cache/vk_gltf_viewer_gb300/autotune.json.
 """
 from __future__ import annotations
@@ -17,6 +18,7 @@ from pathlib import Path
 
 import torch
 
+from . import abi
 from .renderer import DeviceScene, Renderer, ViewBuffers
 
 
@@ -30,6 +32,10 @@ def cache_path() -> Path:
 def device_key(device: int) -> str:
     p = torch.cuda.get_device_properties(device)
     return f"{p.name}|sm{p.multi_processor_count}|cc{p.major}.{p.minor}"
+
+
+def library_key() -> str:
+    return "lib=" + hashlib.sha1(abi.LIB_PATH.read_bytes()).hexdigest()[:12]
 
 
 def workload_key(scene: DeviceScene, views: list[ViewBuffers], flags: int) -> str:
@@ -51,7 +57,7 @@ def tune(r: Renderer, scene: DeviceScene, views: list[ViewBuffers], flags: int, 
     """Returns {"bin_size", "meshlets_per_cta", "table", "cached", "key"} for
     this workload, sweeping (and caching) unless a cached entry exists."""
     path = path or cache_path()
-    key = device_key(r.device) + "||" + workload_key(scene, views, flags)
+    key = "||".join((device_key(r.device), library_key(), workload_key(scene, views, flags)))
     cache = _load(path)
     if not force and key in cache:
         out = dict(cache[key])
