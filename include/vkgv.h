@@ -231,8 +231,8 @@ typedef struct vkgv_graph vkgv_graph;
 
 typedef struct vkgv_config {
     int32_t device;                  /* CUDA device ordinal                       */
-    uint32_t bin_size;               /* raster bin edge in pixels: 8/16/32, 0 = default */
-    uint32_t meshlets_per_cta;       /* meshlets per raster CTA: 1/2/4, 0 = default */
+    uint32_t bin_size;               /* raster bin edge in pixels: 8/16/32/64, 0 = 32 */
+    uint32_t meshlets_per_cta;       /* meshlets in flight per raster CTA: 1/2/4/8, 0 = 1 or 4 by the launch's size */
     uint32_t big_triangle_capacity;  /* binned-triangle queue entries, 0 = default */
     uint32_t spin_limit;             /* bounded device waits, 0 = default         */
     uint32_t _reserved[3];
@@ -340,7 +340,10 @@ int vkgv_graph_kernel_count(const vkgv_graph* graph, uint32_t* out_count);
  * {8, 16, 32} x meshlets per CTA {1, 2, 4}: for each candidate a context
  * built from `base` with those two fields captures this frame as a graph,
  * launches it once to warm up, then `launches` times between CUDA events on
- * a private stream.  The candidates render into the caller's views (every
+ * a private stream.  1 and 4 are the shapes that an untuned context
+ * (meshlets_per_cta = 0) chooses between for each launch, so the one it takes
+ * for this frame is among the candidates; a tuned context keeps its choice for
+ * every launch.  The candidates render into the caller's views (every
  * candidate produces the same visibility; the parity tests cover each).
  * Writes up to entry_capacity entries (in sweep order) and the fastest
  * configuration into *best. */

@@ -1284,13 +1284,11 @@ void launch_raster(const SceneArgs& S, const DeviceView* views, uint32_t nviews,
         // waits for its 4,256 CTAs (84 meshlets: 29.2 -> 32.0 us; 1,152: 30.1 ->
         // 30.4; 64 views of 290: 554.8 -> 551.2), and above 512 views their
         // prefixes leave no room for 28 of them on an SM.  The slow instance
-        // keeps four (1080p 244.1 with one).
-        if (!cfg.warps_per_cta && (uint64_t)S.draw_count * P.nviews >= 16384 && P.nviews <= 512) {
-            launch_variant<1, 4>(P, sm_count, cfg.blocks_per_view, stream);
-            continue;
-        }
-        switch (cfg.warps_per_cta) {
-            case 1: launch_variant<1>(P, sm_count, cfg.blocks_per_view, stream); break;
+        // keeps four (1080p 244.1 with one), also where the caller asks for one,
+        // so that a caller who tries one and four tries both forms of the default.
+        const bool many = (uint64_t)S.draw_count * P.nviews >= 16384 && P.nviews <= 512;
+        switch (cfg.warps_per_cta ? cfg.warps_per_cta : (many ? 1u : 4u)) {
+            case 1: launch_variant<1, 4>(P, sm_count, cfg.blocks_per_view, stream); break;
             case 2: launch_variant<2>(P, sm_count, cfg.blocks_per_view, stream); break;
             case 8: launch_variant<8>(P, sm_count, cfg.blocks_per_view, stream); break;
             default: launch_variant<4>(P, sm_count, cfg.blocks_per_view, stream); break;
