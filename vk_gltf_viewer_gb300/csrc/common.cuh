@@ -270,7 +270,8 @@ __host__ __device__ __forceinline__ bool hiz_second(uint32_t w, uint32_t h, uint
 // -> 132.3 and 552.9 -> 505.0.  Frames of several views share the launch: two
 // spheres of 2048x1100 (2,176) 101.9 -> 101.1, of 2560x1440 132.1 -> 129.1, two
 // torus grids of 2048x1100 1,467 -> 1,443, 16 spheres of it 351.8 -> 343.6.
-inline uint32_t hiz_line(uint32_t nviews) { return nviews == 1 ? 5120u : 2048u; }
+constexpr uint32_t kHizLineOne = 5120, kHizLineMany = 2048;
+inline uint32_t hiz_line(uint32_t nviews) { return nviews == 1 ? kHizLineOne : kHizLineMany; }
 
 __host__ __device__ __forceinline__ int hiz_tile_edge(int level, int top) { return kHizTopTile << (top - level); }
 

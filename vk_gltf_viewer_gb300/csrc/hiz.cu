@@ -23,8 +23,6 @@
 // finish: the footprints of all their columns and rows in one table, the
 // first of them from the top tiled mip in L2, the rest from shared memory
 // with one barrier per level.
-#include <atomic>
-
 #include "kernels.cuh"
 
 namespace vkgv {
@@ -36,13 +34,19 @@ namespace {
 // sizes reaches one texel further per level.
 constexpr int kCap1 = 48, kCap2 = 26, kCap3 = 14, kCap4 = 8;
 constexpr int kThreads = 256;
-// Dynamic shared memory: the tile levels, later reused by the tail's levels
-// when they fit kTailMax floats; the launch sizes it to the larger of the
-// two uses.
+// Dynamic shared memory: the tile levels, later reused by the tail's levels;
+// the launch sizes it to the larger of the two uses.
 constexpr int kOff2 = kCap1 * kCap1, kOff3 = kOff2 + kCap2 * kCap2, kOff4 = kOff3 + kCap3 * kCap3;
 constexpr int kTileFloats = kOff4 + kCap4 * kCap4;
-constexpr int kTailMax = 40960;
-constexpr int kTailAxis = 1024;  // footprint-table entries per axis over all tail levels
+// Footprint-table entries per axis over all tail levels: the first of them is
+// at most 256 wide (level 5 of an edge of 8192), each next one at most half as
+// wide.
+constexpr int kTailAxis = 512;
+static_assert((VKGV_MAX_VIEW_DIM >> (kHizTileLevels + 1)) * 2 <= kTailAxis, "the tail's footprints fit their table");
+// The first tail level has fewer than kHizLineOne texels and each next one at
+// most a quarter of the one below, which stays within what a CTA has without
+// asking for more.
+static_assert((kHizLineOne + kHizLineOne / 3 + 2 * kTailAxis) * 4 + 1024 <= 48 * 1024, "the tail fits shared memory");
 #ifndef VKGV_HIZ_TAIL_BATCH
 #define VKGV_HIZ_TAIL_BATCH 2
 #endif
@@ -345,7 +349,10 @@ __global__ void __launch_bounds__(kThreads, 5) k_hiz(const DeviceView* __restric
         for (uint32_t i = threadIdx.x; i < so + sz; i += kThreads) dst[i] = lv[i];
         first_zero = Lv + 1;
     }
-    // Otherwise each texel reads its footprint from global memory.
+    // The levels with a zero dimension.  (The other branch is the general
+    // reduction, which no accepted view takes; without it the kernel compiles to
+    // 48 registers instead of 40, five CTAs per SM instead of six: 256 views of
+    // 128^2 1,296 -> 1,323 us, held to 40 by its launch bounds 1,300.)
     for (uint32_t j = first_zero; j <= L; ++j) {
         const uint32_t dw = w >> j, dh = h >> j;
         const uint32_t mw = mip_dim(w0, j - 1), mh = mip_dim(h0, j - 1);
@@ -388,19 +395,6 @@ uint32_t tail_floats(uint32_t w, uint32_t h, uint32_t levels) {
 template <bool FIRST>
 void launch_pass(const DeviceView* views, uint32_t nviews, uint32_t tiles_x, uint32_t tiles_y, uint32_t tail,
                  uint32_t line, uint32_t* status, cudaStream_t stream) {
-    // The dynamic shared-memory limit is a per-device function attribute:
-    // set it once for each device a launch runs on (setting it twice is
-    // harmless, so concurrent first launches need no lock).
-    static std::atomic<uint64_t> attr_devices{0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const uint64_t bit = dev < 64 ? (1ull << dev) : 0ull;
-    if (!bit || !(attr_devices.load(std::memory_order_acquire) & bit)) {
-        cudaFuncSetAttribute(k_hiz<FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMax * (int)sizeof(float));
-        attr_devices.fetch_or(bit, std::memory_order_release);
-    }
-    // the tail works in shared memory when all of its levels fit
-    if (tail > (uint32_t)kTailMax) tail = 0;
     const uint32_t floats = tail > (uint32_t)kTileFloats ? tail : (uint32_t)kTileFloats;
     dim3 grid(tiles_x ? tiles_x : 1, tiles_y ? tiles_y : 1, nviews);
     launch_pdl(k_hiz<FIRST>, grid, dim3(kThreads), floats * sizeof(float), stream, views, status, tail, line);
