@@ -462,14 +462,10 @@ struct TriClass {
 // need no clipping.  kFast: snapped, inside the guard band, front-facing,
 // non-zero area, a pixel centre in its bbox, bbox of a fast_size and edge
 // values within int32.
-template <bool SLOW>
 __device__ __forceinline__ int classify(uint32_t i0, uint32_t i1, uint32_t i2, uint32_t vc, const int2* sxy,
                                         const int2* szf, const float4* clip, bool double_sided, float tdet, const RasterCtx& c,
-                                        const RasterQueue& Q, uint32_t d, TriClass& k) {
-    if (i0 >= vc || i1 >= vc || i2 >= vc) {
-        if (!SLOW) report(Q.status, kStatusBadIndex, d);
-        return kDrop;
-    }
+                                        const RasterQueue& Q, TriClass& k) {
+    if (i0 >= vc || i1 >= vc || i2 >= vc) return kDrop;  // reported by the fast instance
     k.q0 = sxy[i0], k.f0 = szf[i0];
     k.q1 = sxy[i1], k.f1 = szf[i1];
     k.q2 = sxy[i2], k.f2 = szf[i2];
@@ -1072,7 +1068,7 @@ __global__ void __launch_bounds__(WARPS * 32, (SLOW ? 16 : VKGV_RASTER_WARPS_PER
                     if (t < tc) {
                         TriClass k;
                         const uint32_t i0 = sidx8[3 * t], i1 = sidx8[3 * t + 1], i2 = sidx8[3 * t + 2];
-                        const int kind = classify<true>(i0, i1, i2, vc, sxy, szf, clip, double_sided, tdet, c, Q, d, k);
+                        const int kind = classify(i0, i1, i2, vc, sxy, szf, clip, double_sided, tdet, c, Q, k);
                         if (kind == kSlowClip) {
                             raster_clipped(clip[i0], clip[i1], clip[i2],
                                            ((uint32_t)(k.f0.y | k.f1.y | k.f2.y) & (OC_ZLO | OC_ZHI)) != 0,
