@@ -246,10 +246,10 @@ __device__ const uint8_t g_bc7_a3b[64] = {
 
 // The interpolation weights of 2-, 3- and 4-bit indices ({0, 21, 43, 64},
 // {0, 9, 18, 27, 37, 46, 55, 64}, {0, 4, 9, 13, 17, 21, 26, 30, 34, 38, 43,
-// 47, 51, 55, 60, 64}) by their arithmetic.
+// 47, 51, 55, 60, 64}) by their arithmetic: of one index (3 or 4 bits), and four
+// at a time below.
 template <int BITS>
 __device__ __forceinline__ uint32_t index_weight(uint32_t i) {
-    if (BITS == 2) return i * 21u + (i >> 1);
     if (BITS == 3) return i * 9u + (i >> 2);
     return (i * 17u + 2u) >> 2;
 }
@@ -629,14 +629,12 @@ constexpr uint8_t kBc6Count[14][13] = {
     {2, 2, 2, 1, 1, 1, 0, 0, 0, 0, 0, 0, 0},  // mode 0x0B
     {2, 2, 2, 1, 1, 1, 0, 0, 0, 0, 0, 0, 0},  // mode 0x0F
 };
-// mode value, transformed, endpoint bits, delta bits R, G, B, regions, tokens
-// (the oracle's stream-order count)
-constexpr uint8_t kBc6Mode[14][8] = {
-    {0x00, 1, 10, 5, 5, 5, 2, 20}, {0x01, 1, 7, 6, 6, 6, 2, 22},   {0x02, 1, 11, 5, 4, 4, 2, 19},
-    {0x06, 1, 11, 4, 5, 4, 2, 21}, {0x0A, 1, 11, 4, 4, 5, 2, 20},  {0x0E, 1, 9, 5, 5, 5, 2, 20},
-    {0x12, 1, 8, 6, 5, 5, 2, 19},  {0x16, 1, 8, 5, 6, 5, 2, 22},   {0x1A, 1, 8, 5, 5, 6, 2, 22},
-    {0x1E, 0, 6, 6, 6, 6, 2, 23},  {0x03, 0, 10, 10, 10, 10, 1, 6}, {0x07, 1, 11, 9, 9, 9, 1, 9},
-    {0x0B, 1, 12, 8, 8, 8, 1, 9},  {0x0F, 1, 16, 4, 4, 4, 1, 9}};
+// Per mode (fields 0x00, 0x01, 0x02, 0x06, .. 0x1E, 0x03, 0x07, 0x0B, 0x0F):
+// transformed, endpoint bits, delta bits R, G, B, regions
+constexpr uint8_t kBc6Mode[14][6] = {
+    {1, 10, 5, 5, 5, 2}, {1, 7, 6, 6, 6, 2}, {1, 11, 5, 4, 4, 2}, {1, 11, 4, 5, 4, 2}, {1, 11, 4, 4, 5, 2},
+    {1, 9, 5, 5, 5, 2}, {1, 8, 6, 5, 5, 2}, {1, 8, 5, 6, 5, 2}, {1, 8, 5, 5, 6, 2}, {0, 6, 6, 6, 6, 2},
+    {0, 10, 10, 10, 10, 1}, {1, 11, 9, 9, 9, 1}, {1, 12, 8, 8, 8, 1}, {1, 16, 4, 4, 4, 1}};
 
 __device__ __forceinline__ int32_t bc6_sext(uint32_t v, uint32_t n) {
     const uint32_t s = 32u - n;
@@ -686,9 +684,9 @@ __device__ __forceinline__ uint32_t bc6_field(const uint4& q) {
 // Channel C of end point E, unquantised to 16 bits.
 template <int MI, int E, int C>
 __device__ __forceinline__ uint32_t bc6_end(const uint4& q, uint32_t base, bool sgn) {
-    constexpr uint32_t bits = kBc6Mode[MI][2], delta = kBc6Mode[MI][3 + C];
+    constexpr uint32_t bits = kBc6Mode[MI][1], delta = kBc6Mode[MI][2 + C];
     uint32_t v = E == 0 ? base : bc6_field<MI, E * 3 + C>(q);
-    if constexpr (E > 0 && kBc6Mode[MI][1] != 0)  // a signed delta to the base end point
+    if constexpr (E > 0 && kBc6Mode[MI][0] != 0)  // a signed delta to the base end point
         v = (base + (uint32_t)bc6_sext(v, delta)) & ((1u << bits) - 1u);
     return (uint32_t)bc6_unquantize(sgn ? bc6_sext(v, bits) : (int32_t)v, bits, sgn) & 0xFFFFu;
 }
@@ -701,7 +699,7 @@ __device__ __forceinline__ void bc6_header(const uint4& q, bool sgn, uint32_t* o
     out[0 * pitch] = bc6_end<MI, 0, 0>(q, b0, sgn) | (bc6_end<MI, 1, 0>(q, b0, sgn) << 16);
     out[1 * pitch] = bc6_end<MI, 0, 1>(q, b1, sgn) | (bc6_end<MI, 1, 1>(q, b1, sgn) << 16);
     out[2 * pitch] = bc6_end<MI, 0, 2>(q, b2, sgn) | (bc6_end<MI, 1, 2>(q, b2, sgn) << 16);
-    if constexpr (kBc6Mode[MI][6] == 2) {
+    if constexpr (kBc6Mode[MI][5] == 2) {
         out[3 * pitch] = bc6_end<MI, 2, 0>(q, b0, sgn) | (bc6_end<MI, 3, 0>(q, b0, sgn) << 16);
         out[4 * pitch] = bc6_end<MI, 2, 1>(q, b1, sgn) | (bc6_end<MI, 3, 1>(q, b1, sgn) << 16);
         out[5 * pitch] = bc6_end<MI, 2, 2>(q, b2, sgn) | (bc6_end<MI, 3, 2>(q, b2, sgn) << 16);
