@@ -566,10 +566,18 @@ __global__ void __launch_bounds__(256, 3) k_diff_shade_chunks(DiffArgs A, const 
     if (BACKWARD && A.loss) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
-        if ((threadIdx.x & 31) == 0) atomicAdd(A.loss, loss_acc);
+        if ((threadIdx.x & 31) == 0) VP[0] = loss_acc;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+        // one addition a CTA: with one a warp the order of 3,648 of them moved the
+        // loss of 64 views of 512^2 by 8.8e-7 of it (standard deviation)
+        if (BACKWARD && A.loss) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) sum += s_vp[w][0];
+            atomicAdd(A.loss, sum);
+        }
         __threadfence();
         if (atomicAdd(work + 1, 1u) == gridDim.x - 1) {
             work[0] = 0;
