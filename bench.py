@@ -1013,7 +1013,7 @@ def main():
                  "unit": "warp instructions/s", "frac": instr / (dom_ms / 1000.0) / peak_issue,
                  "note": "152 SMs x 4 schedulers x 1 warp instruction per cycle at the sampled SM clock; "
                          "instruction count from the ncu capture of profiles/raster_meshlets_c2_1080p.md"}
-    # The L2 atomic bound of the same launch: its 64-bit atomicMax count and
+    # The L2 atomic bound of the same launch: its 64-bit maxima's sectors and
     # the L2 atomic units' busy fraction from the ncu capture, rescaled from
     # the capture's duration to this run's.
     # Whole-frame algorithmic bytes (12 B per draw, 4 B per survivor, the
@@ -1026,7 +1026,7 @@ def main():
                   "unit": "GB/s", "frac": frame_bytes / (ms_per_step / 1000.0) / 1e9 / peak}
     atomic = None
     if dominant == "raster1" and prof_atom and prof_atom_busy is not None and prof_ncu_us and dom_ms > 0:
-        atomic = {"atomics": prof_atom / (prof_meshlets or surv) * surv, "unit": "64-bit atomicMax/s",
+        atomic = {"atomics": prof_atom / (prof_meshlets or surv) * surv, "unit": "sectors of 64-bit max reductions/s",
                   "achieved": prof_atom / (prof_meshlets or surv) * surv / (dom_ms / 1000.0),
                   "frac": prof_atom_busy / 100.0 * prof_ncu_us / (dom_ms * 1000.0),
                   "note": "L2 atomic-unit busy fraction (lts__d_atomic_input_cycles_active) from the ncu capture "

@@ -38,7 +38,7 @@ struct RasterLists {
 struct RasterConfig {
     uint32_t small_area;      // bbox pixel area rasterised inline by the lane
     uint32_t chunk;           // edge of the binned chunk in pixels (8, 16, 32, 64)
-    uint32_t warps_per_cta;   // meshlets in flight per CTA; 0: by the launch's size
+    uint32_t warps_per_cta;   // meshlets in flight per CTA (1: four in the slow instance); 0: 1 or 4 by the launch's size
     uint32_t blocks_per_view;
 };
 

@@ -133,9 +133,9 @@ __device__ __forceinline__ void store_rows(const uint32_t* v, uint32_t* buf, uin
 // BC1-BC5: one thread per block, a warp per 32 blocks of a block row, so that
 // each of its four texel rows is one contiguous 512-byte store.  The codes of
 // four texels pass through the palette's channel planes as byte selectors.
-// Bound by its writes at 0.75-0.89 of the measured copy bandwidth (8192^2:
-// BC1 94.9 -> 53.9 us, BC3 152 -> 64, BC5 146 -> 66; with four lanes per block,
-// one row each, the palette was built four times and looked up per texel).
+// Bound by its writes at 0.83-0.97 of the measured copy bandwidth (8192^2:
+// BC1 94.9 -> 46.0 us, BC3 152 -> 59.4; with four lanes per block, one row each,
+// the palette was built four times and looked up per texel).
 // Where the image's rows are 16-byte words, each lane stores its own: through
 // the warp's buffer whenever a row held fewer than 32 blocks, narrow images were
 // slower than with four lanes per block (BC1 4x16384 3.0 -> 3.5 us, now 2.7; 4x4

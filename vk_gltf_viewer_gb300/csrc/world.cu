@@ -12,8 +12,9 @@
 // ((I * L_root) * ...) * L_node:
 //   k_world_slots  a group of lanes per slot, one lane per node of the path,
 //                  then the product by shuffles;
-//   k_world_local, k_world_chain  deep or large trees (launch_world_transforms
-//                  has the line): one thread per node, then one per slot.
+//   k_world_local, k_world_chain  deep or large trees, and trees whose shared
+//                  nodes have many channels (launch_world_transforms has the
+//                  lines): one thread per node, then one per slot.
 // The draw list is k_world_draws: one block per tile of 1024 draws whose
 // first segment the plan holds, the tile's records staged in shared memory
 // and stored as 16-byte words.
